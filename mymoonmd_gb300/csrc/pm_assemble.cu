@@ -68,6 +68,20 @@ void build_qk_tables(int dim, int k, int qn, RefTables& t) {
   t.xi.assign(size_t(t.nq) * 3, 0.0);
   t.phi.assign(size_t(t.nq) * t.nb, 0.0);
   t.dphi.assign(size_t(3) * t.nq * t.nb, 0.0);
+  t.t1 = Tables1d{};
+  for (int l = 0; l < qn; ++l) {
+    double v[3], d[3];
+    lag1d(k, x1[l], v, d);
+    t.t1.xi[l] = x1[l];
+    for (int i = 0; i < nb1; ++i) {
+      t.t1.phiw[l * nb1 + i] = w1[l] * v[i];
+      for (int j = 0; j < nb1; ++j) {
+        t.t1.M[i * nb1 + j] += w1[l] * v[i] * v[j];
+        t.t1.S[i * nb1 + j] += w1[l] * d[i] * d[j];
+        t.t1.C[i * nb1 + j] += w1[l] * v[i] * d[j];
+      }
+    }
+  }
   int q = 0;
   for (int i = 0; i < (dim == 3 ? qn : 1); ++i)
     for (int j = 0; j < qn; ++j)
@@ -365,6 +379,72 @@ __global__ void __launch_bounds__(256) k_elem_cd(int n_cells, const double* __re
   }
 }
 
+// J^{-T}, its determinant and the reference-tensor coefficients of one affine
+// cell: out[k] = |det J| A_ab (a <= b, A_ab = eps sum_d G_da G_db), then
+// |det J| beta_a (beta_a = sum_d b_d G_da), then |det J| c; returns |det J|
+template <int DIM>
+__device__ __forceinline__ double tensor_coefficients(const double J[3][3], const CdCoef& co, double* out) {
+  double G[3][3] = {{0}}, det;
+  if (DIM == 2) {
+    det = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+    const double r = 1.0 / det;
+    G[0][0] = J[1][1] * r;  G[0][1] = -J[1][0] * r;
+    G[1][0] = -J[0][1] * r; G[1][1] = J[0][0] * r;
+  } else {
+    det = J[0][0] * (J[1][1] * J[2][2] - J[1][2] * J[2][1]) -
+          J[0][1] * (J[1][0] * J[2][2] - J[1][2] * J[2][0]) +
+          J[0][2] * (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
+    const double r = 1.0 / det;
+    G[0][0] = (J[1][1] * J[2][2] - J[1][2] * J[2][1]) * r;
+    G[0][1] = -(J[1][0] * J[2][2] - J[1][2] * J[2][0]) * r;
+    G[0][2] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]) * r;
+    G[1][0] = -(J[0][1] * J[2][2] - J[0][2] * J[2][1]) * r;
+    G[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * r;
+    G[1][2] = -(J[0][0] * J[2][1] - J[0][1] * J[2][0]) * r;
+    G[2][0] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * r;
+    G[2][1] = -(J[0][0] * J[1][2] - J[0][2] * J[1][0]) * r;
+    G[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * r;
+  }
+  const double adet = fabs(det);
+  const double bv[3] = {co.b0, co.b1, co.b2};
+  int k = 0;
+  for (int a = 0; a < DIM; ++a)
+    for (int b = a; b < DIM; ++b) {
+      double s = 0.0;
+      for (int d = 0; d < DIM; ++d) s += G[d][a] * G[d][b];
+      out[k++] = adet * co.eps * s;
+    }
+  for (int a = 0; a < DIM; ++a) {
+    double s = 0.0;
+    for (int d = 0; d < DIM; ++d) s += bv[d] * G[d][a];
+    out[k++] = adet * s;
+  }
+  out[k] = adet * co.c;
+  return adet;
+}
+
+// K_e = sum_k coef_k T_k for the cells of a block: a thread keeps the NT
+// reference-tensor values of one entry in registers and walks the cells, so
+// the tables are read once per block and not once per cell
+template <int NB, int NT>
+__device__ __forceinline__ void tensor_matrices(int nc, const double (*coef)[NT], const double* __restrict__ T,
+                                                double* __restrict__ K) {
+  constexpr int NB2 = NB * NB, TP = NB2 >= 256 ? 256 : NB2, NG = 256 / TP;
+  const int tg = threadIdx.x / TP, tp = threadIdx.x % TP;
+  if (tg >= NG) return;
+  for (int p = tp; p < NB2; p += TP) {
+    double tv[NT];
+#pragma unroll
+    for (int k = 0; k < NT; ++k) tv[k] = __ldg(T + k * NB2 + p);
+    for (int cl = tg; cl < nc; cl += NG) {
+      double s = 0.0;
+#pragma unroll
+      for (int k = 0; k < NT; ++k) s = fma(coef[cl][k], tv[k], s);
+      K[(size_t)cl * NB2 + p] = s;
+    }
+  }
+}
+
 // Reference-tensor element kernel. On an affine cell with cell-constant eps,
 // b, c the quadrature sum of BilinearAssembleGalerkin factors into
 //   K_e = |det J| ( sum_{a<=b} A_ab S_ab + sum_a beta_a C_a + c M ),
@@ -373,66 +453,30 @@ __global__ void __launch_bounds__(256) k_elem_cd(int n_cells, const double* __re
 // computed once per element type). This is the same quadrature applied in a
 // different summation order: NT FMAs per entry instead of 4 per quadrature
 // point. The right-hand side keeps the per-point loop (f varies in the cell).
-template <int DIM, int NB, int NQ, int CHUNK, int NV = DIM == 2 ? 4 : 8>
+// Tetrahedra (P1, P2); quadrilaterals and hexahedra run k_elem_cd_qk.
+template <int NB, int NQ, int CH>
 __global__ void __launch_bounds__(256) k_elem_cd_tensor(int n_cells, const double* __restrict__ verts,
                                                         const double* __restrict__ ref,
                                                         const double* __restrict__ T, CdCoef co,
                                                         double* __restrict__ K, double* __restrict__ F) {
-  constexpr int NT = DIM * (DIM + 1) / 2 + DIM + 1;
-  __shared__ double coef[CHUNK][NT];
-  __shared__ double fq[CHUNK][NQ];
-  __shared__ double geo[CHUNK][13];  // x0, J (row-major), |det J|
+  constexpr int DIM = 3, NV = 4, NT = 10;
+  __shared__ double coef[CH][NT];
+  __shared__ double fq[CH][NQ];
+  __shared__ double geo[CH][13];  // x0, J (row-major), |det J|
   const double* phi = ref;
   const double* w = ref + 4 * NQ * NB;
   const double* xi = w + NQ;
-  const int c0 = blockIdx.x * CHUNK;
-  const int nc = min(CHUNK, n_cells - c0);
+  const int c0 = blockIdx.x * CH;
+  const int nc = min(CH, n_cells - c0);
   const int t = threadIdx.x;
-  double x0[3] = {0, 0, 0}, J[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
-  // per-cell coefficients (one thread per cell)
   if (t < nc) {
+    double x0[3] = {0, 0, 0}, J[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
     affine_map<DIM, NV>(verts + (size_t)(c0 + t) * NV * DIM, x0, J);
-    double G[3][3] = {{0}}, det;
-    if (DIM == 2) {
-      det = J[0][0] * J[1][1] - J[0][1] * J[1][0];
-      const double r = 1.0 / det;
-      G[0][0] = J[1][1] * r;  G[0][1] = -J[1][0] * r;
-      G[1][0] = -J[0][1] * r; G[1][1] = J[0][0] * r;
-    } else {
-      det = J[0][0] * (J[1][1] * J[2][2] - J[1][2] * J[2][1]) -
-            J[0][1] * (J[1][0] * J[2][2] - J[1][2] * J[2][0]) +
-            J[0][2] * (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
-      const double r = 1.0 / det;
-      G[0][0] = (J[1][1] * J[2][2] - J[1][2] * J[2][1]) * r;
-      G[0][1] = -(J[1][0] * J[2][2] - J[1][2] * J[2][0]) * r;
-      G[0][2] = (J[1][0] * J[2][1] - J[1][1] * J[2][0]) * r;
-      G[1][0] = -(J[0][1] * J[2][2] - J[0][2] * J[2][1]) * r;
-      G[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * r;
-      G[1][2] = -(J[0][0] * J[2][1] - J[0][1] * J[2][0]) * r;
-      G[2][0] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * r;
-      G[2][1] = -(J[0][0] * J[1][2] - J[0][2] * J[1][0]) * r;
-      G[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * r;
-    }
-    const double adet = fabs(det);
-    const double bv[3] = {co.b0, co.b1, co.b2};
-    int k = 0;
-    for (int a = 0; a < DIM; ++a)
-      for (int b = a; b < DIM; ++b) {
-        double s = 0.0;
-        for (int d = 0; d < DIM; ++d) s += G[d][a] * G[d][b];
-        coef[t][k++] = adet * co.eps * s;
-      }
-    for (int a = 0; a < DIM; ++a) {
-      double s = 0.0;
-      for (int d = 0; d < DIM; ++d) s += bv[d] * G[d][a];
-      coef[t][k++] = adet * s;
-    }
-    coef[t][k] = adet * co.c;
+    geo[t][12] = tensor_coefficients<DIM>(J, co, coef[t]);
     for (int d = 0; d < 3; ++d) {
       geo[t][d] = x0[d];
       for (int a = 0; a < 3; ++a) geo[t][3 + d * 3 + a] = J[d][a];
     }
-    geo[t][12] = adet;
   }
   __syncthreads();
   // quadrature weights times |det J| times f at the mapped points, one
@@ -448,18 +492,180 @@ __global__ void __launch_bounds__(256) k_elem_cd_tensor(int n_cells, const doubl
     fq[cl][q] = w[q] * geo[cl][12] * rhs_value_pi(co, DIM, x);
   }
   __syncthreads();
-  for (int e = t; e < nc * NB * NB; e += blockDim.x) {
-    const int cl = e / (NB * NB), p = e % (NB * NB);
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < NT; ++k) s = fma(coef[cl][k], __ldg(T + k * NB * NB + p), s);
-    K[(size_t)(c0 + cl) * NB * NB + p] = s;
-  }
+  tensor_matrices<NB, NT>(nc, coef, T, K + (size_t)c0 * NB * NB);
   for (int e = t; e < nc * NB; e += blockDim.x) {
     const int cl = e / NB, i = e % NB;
     double s = 0.0;
     for (int q = 0; q < NQ; ++q) s += fq[cl][q] * phi[q * NB + i];
     F[(size_t)(c0 + cl) * NB + i] = s;
+  }
+}
+
+// Element kernel of the tensor-product elements (Q1, Q2), CH cells per block.
+//
+// FP64 arithmetic bounds it (about 500 G FMA/s on GB300), so the sums are
+// factored by direction wherever the cell allows it:
+//  * cells whose Jacobian has one nonzero per row (edges along the axes, in
+//    any orientation): the reference tensors are products of the 1D matrices
+//    M, S, C and the cross terms vanish, so
+//      K = A0 (x) (M (x) M) + M (x) (A1 (x) M + M (x) A2),
+//      A_a = |det J| (A_aa S + beta_a C)  (+ |det J| c M in A0),
+//    two FMAs per entry instead of NT = 10, and sin / cos of the manufactured
+//    right-hand side at QN points per direction instead of QN^DIM points;
+//  * other affine cells: the reference-tensor sum of tensor_matrices. One
+//    such cell sends its whole block there.
+// The element right-hand side is contracted direction by direction for both
+// (QN^DIM K1 products three times instead of QN^DIM K1^DIM). Eight hexahedra
+// per block: with 64 a block took 185 us, and a 4^3 level (one block) as long
+// as a 16^3 one. Assembly of the 3D Q2 16^3 level (4,096 cells, this kernel
+// and the gather): 224 us with NT FMAs per entry and 64 cells per block, 55 us.
+template <int DIM, int K1, int QN, int CH>
+__global__ void __launch_bounds__(256) k_elem_cd_qk(int n_cells, const double* __restrict__ verts,
+                                                    const double* __restrict__ T, Tables1d tb, CdCoef co,
+                                                    double* __restrict__ K, double* __restrict__ F) {
+  constexpr int N2 = K1 * K1;
+  constexpr int NB = DIM == 2 ? N2 : N2 * K1, NB2 = NB * NB;
+  constexpr int NQ = DIM == 2 ? QN * QN : QN * QN * QN;
+  constexpr int YZ = DIM == 2 ? N2 : N2 * N2;  // (row, column) pairs of the directions above the first
+  constexpr int NT = DIM * (DIM + 1) / 2 + DIM + 1;
+  constexpr int NV = DIM == 2 ? 4 : 8;
+  __shared__ double sM[N2], sS[N2], sC[N2], sPw[QN * K1], sXi[QN];
+  __shared__ double coef[CH][NT];
+  __shared__ double geo[CH][13];  // x0, J (row-major), |det J|
+  __shared__ int axis[CH][3];     // axis-aligned cells: the local direction along space direction d
+  __shared__ double A[CH][DIM][N2];
+  __shared__ double P[YZ], Q[CH][YZ];
+  __shared__ double sc[CH][DIM][QN][2];
+  __shared__ double buf[2][CH * NQ];
+  const int c0 = blockIdx.x * CH;
+  const int nc = min(CH, n_cells - c0);
+  const int t = threadIdx.x;
+  if (t < N2) {
+    sM[t] = tb.M[t];
+    sS[t] = tb.S[t];
+    sC[t] = tb.C[t];
+  }
+  if (t >= 32 && t < 32 + QN * K1) sPw[t - 32] = tb.phiw[t - 32];
+  if (t >= 64 && t < 64 + QN) sXi[t - 64] = tb.xi[t - 64];
+  bool aligned = true;
+  if (t < nc) {
+    double x0[3] = {0, 0, 0}, J[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
+    affine_map<DIM, NV>(verts + (size_t)(c0 + t) * NV * DIM, x0, J);
+    geo[t][12] = tensor_coefficients<DIM>(J, co, coef[t]);
+    for (int d = 0; d < 3; ++d) {
+      geo[t][d] = x0[d];
+      for (int a = 0; a < 3; ++a) geo[t][3 + d * 3 + a] = J[d][a];
+    }
+    for (int d = 0; d < DIM; ++d) {
+      int cnt = 0, at = 0;
+      for (int a = 0; a < DIM; ++a)
+        if (J[d][a] != 0.0) {
+          ++cnt;
+          at = a;
+        }
+      axis[t][d] = at;
+      aligned = aligned && cnt == 1;
+    }
+  }
+  const bool tensor = __syncthreads_and(aligned) != 0;
+  // the sine right-hand side needs its 1D values only
+  const bool sine1d = tensor && co.manufactured == 1;
+  if (sine1d)
+    for (int e = t; e < nc * DIM * QN; e += 256) {
+      const int cl = e / (DIM * QN), d = (e / QN) % DIM, q = e % QN;
+      const double x = geo[cl][d] + geo[cl][3 + d * 3 + axis[cl][d]] * sXi[q];
+      sincospi(x, &sc[cl][d][q][0], &sc[cl][d][q][1]);
+    }
+  if (tensor) {
+    for (int e = t; e < nc * DIM * N2; e += 256) {
+      const int cl = e / (DIM * N2), a = (e / N2) % DIM, k = e % N2;
+      // a == b terms sit at 0, DIM, 2 DIM - 1 of the (a, b) list
+      const double s = coef[cl][a == 0 ? 0 : a == 1 ? DIM : 2 * DIM - 1];
+      double v = s * sS[k] + coef[cl][DIM * (DIM + 1) / 2 + a] * sC[k];
+      if (a == 0) v += coef[cl][NT - 1] * sM[k];
+      A[cl][a][k] = v;
+    }
+  }
+  __syncthreads();
+  if (tensor) {
+    for (int e = t; e < YZ; e += 256) P[e] = DIM == 2 ? sM[e] : sM[e / N2] * sM[e % N2];
+    for (int e = t; e < nc * YZ; e += 256) {
+      const int cl = e / YZ, k = e % YZ;
+      Q[cl][k] = DIM == 2 ? A[cl][1][k] : A[cl][1][k / N2] * sM[k % N2] + sM[k / N2] * A[cl][DIM - 1][k % N2];
+    }
+  }
+  // f at the quadrature points
+  const double pi = 3.14159265358979323846;
+  for (int e = t; e < nc * NQ; e += 256) {
+    const int cl = e / NQ, q = e % NQ;
+    const int ql[3] = {q % QN, (q / QN) % QN, q / (QN * QN)};
+    double f;
+    if (sine1d) {
+      double s[3], c[3];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        const int a = axis[cl][d];
+        const int qa = a == 0 ? ql[0] : a == 1 ? ql[1] : ql[2];
+        s[d] = sc[cl][d][qa][0];
+        c[d] = sc[cl][d][qa][1];
+      }
+      const double e0 = DIM * co.eps * pi * pi + co.c;
+      if (DIM == 2) {
+        f = e0 * (s[0] * s[1]) + pi * (co.b0 * c[0] * s[1] + co.b1 * s[0] * c[1]);
+      } else {
+        const double s12 = s[1] * s[2];
+        f = e0 * (s[0] * s12) +
+            pi * (co.b0 * c[0] * s12 + s[0] * (co.b1 * c[1] * s[2] + co.b2 * s[1] * c[2]));
+      }
+    } else {
+      double x[3] = {0.0, 0.0, 0.0};
+      for (int d = 0; d < DIM; ++d) {
+        double s = geo[cl][d];
+        for (int a = 0; a < DIM; ++a) s += geo[cl][3 + d * 3 + a] * sXi[ql[a]];
+        x[d] = s;
+      }
+      f = rhs_value_pi(co, DIM, x);
+    }
+    buf[0][cl * NQ + q] = f;
+  }
+  __syncthreads();
+  // F_i = |det J| sum_q w_q f(x_q) phi_i(q), direction by direction: in
+  // [points of the directions above][QN][basis indices already made], out
+  // [..][K1][..]
+  int rest = DIM == 2 ? QN : QN * QN, done = 1, in = 0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const int per = rest * K1 * done;  // outputs per cell
+    for (int e = t; e < nc * per; e += 256) {
+      const int cl = e / per, r = e % per;
+      // the basis indices of the finished directions are kept innermost
+      const int lo = r % done, i = (r / done) % K1, hi = r / (done * K1);
+      const double* src = buf[in] + cl * NQ + hi * QN * done + lo;
+      double s = 0.0;
+#pragma unroll
+      for (int q = 0; q < QN; ++q) s = fma(sPw[q * K1 + i], src[q * done], s);
+      if (d == DIM - 1) F[(size_t)(c0 + cl) * NB + r] = s * geo[cl][12];
+      else buf[in ^ 1][cl * NQ + r] = s;
+    }
+    in ^= 1;
+    done *= K1;
+    rest /= QN;
+    __syncthreads();
+  }
+  double* Kc = K + (size_t)c0 * NB2;
+  if (!tensor) {
+    tensor_matrices<NB, NT>(nc, coef, T, Kc);
+    return;
+  }
+  constexpr int TP = NB2 >= 256 ? 256 : NB2, NG = 256 / TP;
+  const int tg = t / TP, tp = t % TP;
+  if (tg >= NG) return;
+  for (int p = tp; p < NB2; p += TP) {
+    const int i = p / NB, j = p % NB;
+    const int x = (i % K1) * K1 + j % K1, y = ((i / K1) % K1) * K1 + (j / K1) % K1;
+    const int yz = DIM == 2 ? y : y * N2 + (i / N2) * K1 + j / N2;
+    const double m = sM[x], pv = P[yz];
+    for (int cl = tg; cl < nc; cl += NG) Kc[(size_t)cl * NB2 + p] = fma(A[cl][0][x], pv, m * Q[cl][yz]);
   }
 }
 
@@ -495,29 +701,63 @@ void build_ref_tensors(const RefTables& t, std::vector<double>& out) {
     }
 }
 
-template <int DIM, int NB, int NQ, int NV = DIM == 2 ? 4 : 8>
-static void launch_elem_tensor(pm_ctx* c, int n_cells, const double* verts, const double* ref,
-                               const double* T, const CdCoef& co, double* K, double* F) {
-  constexpr int CHUNK = 64;
-  const int grid = (n_cells + CHUNK - 1) / CHUNK;
-  k_elem_cd_tensor<DIM, NB, NQ, CHUNK, NV><<<grid, 256, 0, c->stream>>>(n_cells, verts, ref, T, co, K, F);
+template <int NB, int NQ>
+static void launch_elem_tensor(pm_ctx* c, int n_cells, const double* verts, const double* ref, const double* T,
+                               const CdCoef& co, double* K, double* F) {
+  constexpr int CH = 32;
+  k_elem_cd_tensor<NB, NQ, CH>
+      <<<(n_cells + CH - 1) / CH, 256, 0, c->stream>>>(n_cells, verts, ref, T, co, K, F);
   PM_CHECK_LAUNCH();
   c->kernel_launches++;
 }
 
-// stage 2: CSR values from the element matrices, in cell order
-__global__ void k_gather(int nnz, const int* __restrict__ ptr, const int* __restrict__ idx,
-                         const double* __restrict__ K, double* __restrict__ vals) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int t = ptr[e]; t < ptr[e + 1]; ++t) s += K[idx[t]];
-    vals[e] = s;
-  }
+// cells per block: about 6,000 matrix entries per block (few enough that the
+// 64 cells of a 4^3 level still spread over 8 blocks)
+template <int DIM, int K1, int QN>
+static void launch_elem_qk(pm_ctx* c, int n_cells, const double* verts, const DevRefTables& rt, const CdCoef& co,
+                           double* K, double* F) {
+  constexpr int CH = DIM == 3 ? (K1 == 3 ? 8 : 32) : (K1 == 3 ? 32 : 64);
+  k_elem_cd_qk<DIM, K1, QN, CH>
+      <<<(n_cells + CH - 1) / CH, 256, 0, c->stream>>>(n_cells, verts, rt.tensors.p, rt.t1, co, K, F);
+  PM_CHECK_LAUNCH();
+  c->kernel_launches++;
 }
 
-__global__ void k_set_unit(int n, const int* __restrict__ pos, double* __restrict__ vals) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) vals[pos[i]] = 1.0;
+// Stage 2: CSR values and right-hand side from the element matrices and
+// vectors, each entry summing its contributions in cell order. An entry
+// without contributions is a Dirichlet row's diagonal (1) or right-hand side
+// (0). Four index loads and then four value loads of an entry are in flight
+// at a time; one launch for the matrix and the right-hand side (three with a
+// pass for the unit diagonals). Bound by the scattered reads of the element
+// matrices.
+__device__ __forceinline__ double gather_entry(const int* __restrict__ idx, const double* __restrict__ K, int beg,
+                                               int end) {
+  constexpr int U = 4;
+  double s = 0.0;
+  for (int t = beg; t < end; t += U) {
+    int k[U];
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) k[u] = t + u < end ? __ldg(idx + t + u) : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = k[u] >= 0 ? __ldg(K + k[u]) : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t + u < end) s += v[u];
+  }
+  return s;
+}
+
+__global__ void __launch_bounds__(256) k_gather(int nnz, const int* __restrict__ ptr, const int* __restrict__ idx,
+                                                const double* __restrict__ K, double* __restrict__ vals, int n,
+                                                const int* __restrict__ rptr, const int* __restrict__ ridx,
+                                                const double* __restrict__ F, double* __restrict__ rhs) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+    const int beg = __ldg(ptr + e), end = __ldg(ptr + e + 1);
+    vals[e] = beg < end ? gather_entry(idx, K, beg, end) : 1.0;
+  }
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
+    rhs[e] = gather_entry(ridx, F, __ldg(rptr + e), __ldg(rptr + e + 1));
 }
 
 template <int DIM, int NB, int NQ, int CPB, int NV = DIM == 2 ? 4 : 8>
@@ -831,7 +1071,6 @@ void DevAssemblyLevel::upload(pm_ctx* c, const DiscLevel& L, int dim, int nvc) {
   gat_idx.upload(L.gat_idx, c->stream);
   rgat_ptr.upload(L.rgat_ptr, c->stream);
   rgat_idx.upload(L.rgat_idx, c->stream);
-  diag_pos.upload(L.diag_pos, c->stream);
   nm_dof.upload(L.nm_dof, c->stream);
   nm_ptr.upload(L.nm_ptr, c->stream);
   nm_cell.upload(L.nm_cell, c->stream);
@@ -855,18 +1094,18 @@ void launch_cd_elements(pm_ctx* c, const DevAssemblyLevel& L, int dim, int k, in
   const CdCoef co = make_coef(cf);
   const double* T = rt.tensors.p;
   if (!c->assembly_quadrature_loop && T) {
-    if (dim == 2 && k == 1 && qn == 3) launch_elem_tensor<2, 4, 9>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (dim == 2 && k == 1 && qn == 2) launch_elem_tensor<2, 4, 4>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (dim == 2 && k == 2 && qn == 3) launch_elem_tensor<2, 9, 9>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (dim == 2 && k == 2 && qn == 4) launch_elem_tensor<2, 9, 16>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (dim == 3 && k == 1 && qn == 2) launch_elem_tensor<3, 8, 8>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (dim == 3 && k == 1 && qn == 3) launch_elem_tensor<3, 8, 27>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (dim == 3 && k == 2 && qn == 3) launch_elem_tensor<3, 27, 27>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (dim == 3 && k == 2 && qn == 4) launch_elem_tensor<3, 27, 64>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (k == 11 && qn == 11) launch_elem_tensor<3, 4, 11, 4>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (k == 11 && qn == 15) launch_elem_tensor<3, 4, 15, 4>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (k == 12 && qn == 11) launch_elem_tensor<3, 10, 11, 4>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
-    else if (k == 12 && qn == 15) launch_elem_tensor<3, 10, 15, 4>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
+    if (dim == 2 && k == 1 && qn == 3) launch_elem_qk<2, 2, 3>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (dim == 2 && k == 1 && qn == 2) launch_elem_qk<2, 2, 2>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (dim == 2 && k == 2 && qn == 3) launch_elem_qk<2, 3, 3>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (dim == 2 && k == 2 && qn == 4) launch_elem_qk<2, 3, 4>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (dim == 3 && k == 1 && qn == 2) launch_elem_qk<3, 2, 2>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (dim == 3 && k == 1 && qn == 3) launch_elem_qk<3, 2, 3>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (dim == 3 && k == 2 && qn == 3) launch_elem_qk<3, 3, 3>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (dim == 3 && k == 2 && qn == 4) launch_elem_qk<3, 3, 4>(c, L.n_cells, L.verts.p, rt, co, K, F);
+    else if (k == 11 && qn == 11) launch_elem_tensor<4, 11>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
+    else if (k == 11 && qn == 15) launch_elem_tensor<4, 15>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
+    else if (k == 12 && qn == 11) launch_elem_tensor<10, 11>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
+    else if (k == 12 && qn == 15) launch_elem_tensor<10, 15>(c, L.n_cells, L.verts.p, rt.data.p, T, co, K, F);
     else throw Error(PM_E_UNSUPPORTED, "element / quadrature combination not compiled");
   } else if (dim == 2 && k == 1 && qn == 3) launch_elem<2, 4, 9, 16>(c, L.n_cells, L.verts.p, rt.data.p, co, K, F);
   else if (dim == 2 && k == 1 && qn == 2) launch_elem<2, 4, 4, 16>(c, L.n_cells, L.verts.p, rt.data.p, co, K, F);
@@ -883,24 +1122,21 @@ void launch_cd_elements(pm_ctx* c, const DevAssemblyLevel& L, int dim, int k, in
   else throw Error(PM_E_UNSUPPORTED, "element / quadrature combination not compiled");
 }
 
+void gather_cd_level(pm_ctx* c, const DevAssemblyLevel& L, int nnz, const double* K, const double* F, double* vals,
+                     double* rhs) {
+  const int n = L.n_dofs;
+  const int grid = std::max(1, std::min((std::max(nnz, n) + 255) / 256, c->num_sms * 16));
+  k_gather<<<grid, 256, 0, c->stream>>>(nnz, L.gat_ptr.p, L.gat_idx.p, K, vals, n, L.rgat_ptr.p, L.rgat_idx.p, F,
+                                        rhs);
+  PM_CHECK_LAUNCH();
+  c->kernel_launches++;
+}
+
 void assemble_cd_level(pm_ctx* c, const DevAssemblyLevel& L, int dim, int elem, int qn,
                        const pm_cd_coeffs& cf, const DevRefTables& rt, DevCsr& A, double* rhs,
                        double* K, double* F) {
   launch_cd_elements(c, L, dim, elem, qn, cf, rt, K, F);
-  const int nnz = int(A.nnz);
-  k_gather<<<std::max(1, std::min((nnz + 255) / 256, c->num_sms * 16)), 256, 0, c->stream>>>(
-      nnz, L.gat_ptr.p, L.gat_idx.p, K, A.vals.p);
-  PM_CHECK_LAUNCH();
-  const int nd = int(L.diag_pos.n);
-  if (nd) {
-    k_set_unit<<<(nd + 255) / 256, 256, 0, c->stream>>>(nd, L.diag_pos.p, A.vals.p);
-    PM_CHECK_LAUNCH();
-  }
-  const int n = L.n_dofs;
-  k_gather<<<std::max(1, std::min((n + 255) / 256, c->num_sms * 16)), 256, 0, c->stream>>>(
-      n, L.rgat_ptr.p, L.rgat_idx.p, F, rhs);
-  PM_CHECK_LAUNCH();
-  c->kernel_launches += nd ? 3 : 2;
+  gather_cd_level(c, L, int(A.nnz), K, F, A.vals.p, rhs);
   launch_dirichlet_values(c, L, cf, rhs);
   launch_neumann_values(c, L, cf, rhs);
   A.values_changed(c);
@@ -920,6 +1156,7 @@ void DevRefTables::upload(pm_ctx* c, const RefTables& t) {
   build_ref_tensors(t, tens);
   tensors.upload(tens, c->stream);
   nt = n_ref_tensors(t.dim);
+  t1 = t.t1;
 }
 
 }  // namespace pm
@@ -1020,20 +1257,7 @@ extern "C" int pm_assemble_cd_noalloc(pm_problem* p, int level, const pm_cd_coef
     double* F = scratch + kn;
     const pm::Disc& D = *p->disc->d;
     pm::launch_cd_elements(c, L, D.dim(), D.elem, p->qn, coeffs ? *coeffs : p->coeffs, p->ref, K, F);
-    const int nnz = int(p->mats[level]->csr.nnz);
-    pm::k_gather<<<std::max(1, std::min((nnz + 255) / 256, c->num_sms * 16)), 256, 0, c->stream>>>(
-        nnz, L.gat_ptr.p, L.gat_idx.p, K, vals_dev);
-    const int nd = int(L.diag_pos.n);
-    if (nd) pm::k_set_unit<<<(nd + 255) / 256, 256, 0, c->stream>>>(nd, L.diag_pos.p, vals_dev);
-    const int n = L.n_dofs;
-    pm::k_gather<<<std::max(1, std::min((n + 255) / 256, c->num_sms * 16)), 256, 0, c->stream>>>(
-        n, L.rgat_ptr.p, L.rgat_idx.p, F, rhs_dev);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      c->last_error = std::string("kernel launch failed: ") + cudaGetErrorString(e);
-      return PM_E_CUDA;
-    }
-    c->kernel_launches += nd ? 3 : 2;
+    pm::gather_cd_level(c, L, int(p->mats[level]->csr.nnz), K, F, vals_dev, rhs_dev);
     pm::launch_dirichlet_values(c, L, coeffs ? *coeffs : p->coeffs, rhs_dev);
     pm::launch_neumann_values(c, L, coeffs ? *coeffs : p->coeffs, rhs_dev);
     return PM_OK;

@@ -8,9 +8,17 @@
 namespace pm {
 
 // reference-element tables of a Qk element on a tensor Gauss rule
+// 1D tables of a tensor-product element (Q1, Q2) on its Gauss rule, K1 = k + 1
+// basis functions: M_ij = sum_q w phi_i phi_j, S_ij = sum_q w phi_i' phi_j',
+// C_ij = sum_q w phi_i phi_j' (row-major K1 x K1), phiw[q K1 + i] = w_q phi_i(q)
+// and the points
+struct Tables1d {
+  double M[9], S[9], C[9], phiw[12], xi[4];
+};
 struct RefTables {
   int dim = 0, nb = 0, nq = 0;
   std::vector<double> w, xi, phi, dphi;
+  Tables1d t1{};  // quadrilaterals and hexahedra
 };
 void build_qk_tables(int dim, int k, int qn, RefTables& t);
 // P1 (elem 11) / P2 (elem 12) on a tetrahedral rule of qn = 11 or 15 points
@@ -26,6 +34,7 @@ struct DevRefTables {
   // of the reference element): stiffness S_ab (a<=b, S_ab+S_ba for a<b),
   // convection C_a[i][j] = sum_q w phi_i d_a phi_j, mass M; nt x nb x nb
   DBuf<double> tensors;
+  Tables1d t1{};
   void upload(pm_ctx* c, const RefTables& t);
 };
 // number of reference tensors: dim*(dim+1)/2 + dim + 1
@@ -37,7 +46,7 @@ struct DevAssemblyLevel {
   int n_cells = 0, nloc = 0, n_dofs = 0, n_active = 0;
   DBuf<double> verts;
   DBuf<double> bnd_xyz;  // coordinates of the non-active DOFs (3 per DOF)
-  DBuf<int> gat_ptr, gat_idx, rgat_ptr, rgat_idx, diag_pos;
+  DBuf<int> gat_ptr, gat_idx, rgat_ptr, rgat_idx;
   DBuf<int> nm_dof, nm_ptr, nm_cell, nm_code;  // Neumann boundary integral plan
   void upload(pm_ctx* c, const DiscLevel& L, int dim, int nvc);
   void scratch_sizes(size_t& k_elems, size_t& f_elems) const;
@@ -69,6 +78,10 @@ void launch_cd_errors(pm_ctx* c, int dim, int k, int qn, int n_cells, const doub
 // the kernel the context's assembly_quadrature_loop option selects
 void launch_cd_elements(pm_ctx* c, const DevAssemblyLevel& L, int dim, int k, int qn,
                         const pm_cd_coeffs& cf, const DevRefTables& rt, double* K, double* F);
+
+// CSR values and right-hand side of one level from K and F
+void gather_cd_level(pm_ctx* c, const DevAssemblyLevel& L, int nnz, const double* K, const double* F, double* vals,
+                     double* rhs);
 
 // assemble matrix values and right-hand side of one level; K and F are scratch
 // arrays of n_cells*nloc*nloc and n_cells*nloc doubles
