@@ -89,10 +89,10 @@ int pm_ctx_set_option(pm_ctx* c, const char* key, int value) {
     c->sell_shape64 = value;
     return PM_OK;
   }
+  // the launch shape of an earlier coarse factorisation: checked, without effect
   if (std::string(key) == "coarse_cluster") {
     if (value != 1 && value != 2 && value != 4 && value != 8)
       return fail(c, PM_E_INVALID, "coarse_cluster is 1, 2, 4 or 8");
-    c->coarse_cluster = value;
     return PM_OK;
   }
   if (std::string(key) == "sliced_min_entries") {
@@ -103,7 +103,6 @@ int pm_ctx_set_option(pm_ctx* c, const char* key, int value) {
   if (std::string(key) == "coarse_threads") {
     if (value != 0 && value != 256 && value != 512 && value != 1024)
       return fail(c, PM_E_INVALID, "coarse_threads is 0, 256, 512 or 1024");
-    c->coarse_threads = value;
     return PM_OK;
   }
   if (std::string(key) == "jacobi_zero_start") {

@@ -840,17 +840,20 @@ void sor_sweep32(pm_ctx* c, const DevCsr& A, const SorColours& col, const float*
 }
 
 // ------------------------------------------------------- dense inverse ------
-__global__ void k_dense_fill(int na, const int* __restrict__ act, const int* __restrict__ pos,
-                             const int* __restrict__ rp, const int* __restrict__ ci,
-                             const double* __restrict__ v, double* __restrict__ M) {
-  int ia = blockIdx.x * blockDim.x + threadIdx.x;
+// the active block as a dense row-major matrix, one warp per row
+template <class T>
+__global__ void __launch_bounds__(256) k_dense_fill(int na, const int* __restrict__ act, const int* __restrict__ pos,
+                                                    const int* __restrict__ rp, const int* __restrict__ ci,
+                                                    const double* __restrict__ v, T* __restrict__ M) {
+  const int ia = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (ia >= na) return;
   const int i = act[ia];
-  double* row = M + (size_t)ia * na;
-  for (int j = 0; j < na; ++j) row[j] = 0.0;
-  for (int k = rp[i]; k < rp[i + 1]; ++k) {
+  T* row = M + (size_t)ia * na;
+  for (int j = lane; j < na; j += 32) row[j] = T(0);
+  __syncwarp();
+  for (int k = rp[i] + lane; k < rp[i + 1]; k += 32) {
     const int jp = pos[ci[k]];
-    if (jp >= 0) row[jp] = v[k];
+    if (jp >= 0) row[jp] = T(v[k]);
   }
 }
 
@@ -1022,291 +1025,281 @@ __global__ void __launch_bounds__(256) k_gj_coop(int na, double* __restrict__ M,
   }
 }
 
-// (value, position) arg-max with the pivot rule of k_gj_pivot: the largest
-// |a|, the smallest position on ties; NaN never wins
-__device__ __forceinline__ void gj_merge(double& v, int& i, double v2, int i2) {
-  if (v2 > v || (v2 == v && i2 < i)) {
-    v = v2;
-    i = i2;
+// Arg-max with the pivot rule of k_gj_pivot (the largest |a|, the smallest
+// position on ties, NaN never) on the bits of |a| as integers: three warp
+// reductions of 32-bit words. Compared as FP64 numbers in shuffle steps, the
+// search took longer than the elimination step (FP64 compares run on the FP64
+// pipe too).
+__device__ __forceinline__ unsigned long long gj_key(double a) {
+  const unsigned long long k = (unsigned long long)__double_as_longlong(fabs(a));
+  return k > 0x7ff0000000000000ull ? 0ull : k;
+}
+__device__ __forceinline__ unsigned long long gj_key(float a) {
+  const unsigned k = __float_as_uint(fabsf(a));
+  return k > 0x7f800000u ? 0ull : (unsigned long long)k;
+}
+template <bool WIDE>  // WIDE: 64-bit keys
+__device__ __forceinline__ void gj_warp_best(unsigned long long& key, int& pos, int none) {
+  if (WIDE) {
+    const unsigned hi = unsigned(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? unsigned(key) : 0u);
+    const unsigned long long best = ((unsigned long long)mh << 32) | ml;
+    pos = __reduce_min_sync(0xffffffffu, key == best ? pos : none);
+    key = best;
+  } else {
+    const unsigned best = __reduce_max_sync(0xffffffffu, unsigned(key));
+    pos = __reduce_min_sync(0xffffffffu, unsigned(key) == best ? pos : none);
+    key = best;
   }
 }
 
-__device__ __forceinline__ void gj_warp_argmax(double& v, int& i) {
+// Blocked Gauss-Jordan inverse with partial pivoting, in panels of NB columns K:
+// two launches per panel, the matrix before and after a panel in two buffers.
+//
+// k_gj_panel: one block runs the NB elimination steps on the panel's columns of
+// the rows that can still be pivots (position k0 on). Every thread keeps RPT
+// rows of the panel in registers; a step takes two block barriers (the arg-max
+// over the warps' candidates; the scaled pivot row and the row it displaces
+// through shared memory). It leaves D = P^-1 (P: the pivot rows' block of the
+// panel), prm = the row at every position after the panel's swaps, and rowsrc =
+// the composition of all swaps so far.
+// k_gj_apply, on all SMs: the panel's columns become D in the panel's rows and W
+// elsewhere (W = -M_K D, by the panel's elimination steps on every row: formed
+// from D itself it loses accuracy with the condition of P), the others src(prm)
+// (panel rows: 0) + (D | W) * (pivot rows of src); after the last panel the
+// columns go where the row swaps belong in the inverse (out[i][rowsrc[j]]).
+//
+// The chain of columns bounds it. A thread-block cluster with one cluster
+// barrier and one remote row per column took 4 to 8 us per column.
+// Update of a two-level solver (the rest of it takes about 85 us), cluster or
+// row-resident kernel before and now: 225 rows 1,444 and 496 us in FP64, 901 and
+// 304 in FP32; 343 rows 2,977 and 893, 1,763 and 444; 729 rows 6,868 and 3,449
+// in FP64; 1,331 rows 20.8 and 13.7 ms; 2,197 rows (column by column) 190 and 48.
+constexpr int kGjMaxRows = 4096;
+
+template <class T, int NB, int RPT>
+__global__ void __launch_bounds__(1024) k_gj_panel(int n, int k0, int nb, const T* __restrict__ M, T* __restrict__ D,
+                                                   T* __restrict__ steps, int* __restrict__ prm, int* __restrict__ rowsrc,
+                                                   int* __restrict__ flag) {
+  constexpr bool WIDE = sizeof(T) == 8;
+  // by the parity of the step: the warps' candidates (key, position, row) and
+  // the row at the step's position
+  __shared__ __align__(16) T cand[2][32][NB], orow[2][NB];
+  __shared__ unsigned long long wkey[2][32];
+  __shared__ int wpos[2][32];
+  extern __shared__ int sp[];  // row at each position
+  const int t = threadIdx.x, bd = blockDim.x, lane = t & 31, warp = t >> 5, nw = bd >> 5;
+  pdl_enter();
+  T row[RPT][NB];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-    const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-    gj_merge(v, i, v2, i2);
-  }
-}
-
-// Gauss-Jordan inverse with the rows resident in shared memory: block b owns
-// positions [b R, b R + R). One grid barrier per column: after step k every
-// block publishes its best pivot candidate for column k+1 (the arg-max value,
-// the position and the whole row) and the owner of position k+1 publishes that
-// row; at step k+1 every block picks the same pivot from the published
-// candidates, reads the pivot row and the old row k+1 from the published
-// copies and eliminates its own rows in shared memory. The operations per
-// entry are those of k_gj_pivot + k_gj_update, so the inverse is identical.
-__global__ void __launch_bounds__(256) k_gj_rows(int na, int R, double* __restrict__ M, int* __restrict__ perm,
-                                                 double* __restrict__ pub_rows, double* __restrict__ pub_v,
-                                                 int* __restrict__ pub_i, int* __restrict__ flag) {
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
-  extern __shared__ double gj_smem[];
-  __shared__ double s_f[32];  // multipliers of the own rows (R <= 32)
-  __shared__ double wv[8];
-  __shared__ int wi[8];
-  __shared__ int s_p, s_src, s_cand;
-  __shared__ double s_pv;
-  const int t = threadIdx.x, nb = gridDim.x, b = blockIdx.x;
-  const int lane = t & 31, warp = t >> 5;
-  const int r0 = min(na, b * R), r1 = min(na, r0 + R), nr = r1 - r0;
-  double* own = gj_smem;                 // [R][na]
-  double* prow = own + (size_t)R * na;   // scaled pivot row of the step
-  double* orow = prow + na;              // row k before the step
-  const size_t slot = (size_t)(nb + 1) * na;
-  for (int e = t; e < nr * na; e += blockDim.x) own[e] = M[(size_t)r0 * na + e];
-  __syncthreads();
-  // candidates of column col (positions >= col) into buffer buf
-  auto publish = [&](int col, int buf) {
-    if (warp == 0) {
-      double v = -1.0;
-      int i = na;
-      if (lane < nr && r0 + lane >= col) {
-        const double a = fabs(own[(size_t)lane * na + col]);
-        if (a > v) {
-          v = a;
-          i = r0 + lane;
-        }
-      }
-      gj_warp_argmax(v, i);
-      if (lane == 0) {
-        pub_v[buf * nb + b] = v;
-        pub_i[buf * nb + b] = i;
-        s_cand = i < na ? i - r0 : -1;
-      }
-    }
-    __syncthreads();
-    double* out = pub_rows + buf * slot;
-    if (s_cand >= 0)
-      for (int j = t; j < na; j += blockDim.x) out[(size_t)b * na + j] = own[(size_t)s_cand * na + j];
-    if (col >= r0 && col < r1)
-      for (int j = t; j < na; j += blockDim.x) out[(size_t)nb * na + j] = own[(size_t)(col - r0) * na + j];
-  };
-  publish(0, 0);
-  grid.sync();
-  for (int k = 0; k < na; ++k) {
-    const int buf = k & 1;
-    const double* pub = pub_rows + buf * slot;
-    {  // the pivot: the same reduction in every block
-      double v = -1.0;
-      int i = na;
-      for (int q = t; q < nb; q += blockDim.x) gj_merge(v, i, pub_v[buf * nb + q], pub_i[buf * nb + q]);
-      gj_warp_argmax(v, i);
-      if (lane == 0) {
-        wv[warp] = v;
-        wi[warp] = i;
-      }
-      __syncthreads();
-      if (t == 0) {
-        double best = wv[0];
-        int bi = wi[0];
-        for (int w = 1; w < int(blockDim.x >> 5); ++w) gj_merge(best, bi, wv[w], wi[w]);
-        const bool singular = !(best > 0.0);
-        s_p = singular ? k : bi;
-        s_src = singular ? nb : bi / R;
-        s_pv = singular ? 1.0 : pub[(size_t)(bi / R) * na + k];
-        if (b == 0) {
-          perm[k] = s_p;
-          if (singular) *flag = 1;
-        }
-      }
-      __syncthreads();
-    }
-    const int p = s_p;
-    const double pv = s_pv;
-    const double* src = pub + (size_t)s_src * na;
-    const double* old = pub + (size_t)nb * na;
-    for (int j = t; j < na; j += blockDim.x) {
-      prow[j] = (j == k ? 1.0 : src[j]) / pv;
-      orow[j] = old[j];
-    }
-    if (t < nr) {
-      const int i = r0 + t;
-      s_f[t] = (i == p && p != k) ? old[k] : own[(size_t)t * na + k];
-    }
-    __syncthreads();
-    for (int e = t; e < nr * na; e += blockDim.x) {
-      const int ii = e / na, j = e - ii * na;
-      const int i = r0 + ii;
-      double* Mi = own + (size_t)ii * na;
-      if (i == k) {
-        Mi[j] = prow[j];
-      } else {
-        const double base = (i == p && p != k) ? orow[j] : Mi[j];
-        Mi[j] = (j == k ? 0.0 : base) - s_f[ii] * prow[j];
-      }
-    }
-    __syncthreads();
-    if (k + 1 < na) publish(k + 1, buf ^ 1);
-    grid.sync();
-  }
-  for (int e = t; e < nr * na; e += blockDim.x) M[(size_t)r0 * na + e] = own[e];
-}
-
-constexpr size_t kGjRowsSmem = 160 * 1024;  // dynamic shared memory cap of k_gj_rows
-
-// Gauss-Jordan inverse in FP32 on one cluster of CS thread blocks (CS = 1: a
-// single block): block r keeps positions [r R, r R + R) in its shared memory.
-// Per column one cluster barrier. Before it, every block pushes its pivot
-// candidate for the next column (arg-max value and position) into every
-// block's candidate table, keeps the candidate row in its own double-buffered
-// publication slot, and the owner of the next position pushes that row into
-// every block's old-row buffer. After it, every block picks the pivot from its
-// local table (the rule of k_gj_pivot: largest |a|, smallest position on
-// ties), reads the pivot row from the winner's slot (the one remote read of
-// the step) and eliminates its own rows, thread tx on column tx for the rows
-// ty, ty + G, ... . The column swaps are undone on the rows in shared memory
-// before they are written out.
-constexpr int kGjCluster = 8;
-constexpr size_t kGjClusterSmem = 220 * 1024;
-
-template <class T>
-__device__ __forceinline__ void gj_merge(T& v, int& i, T v2, int i2) {
-  if (v2 > v || (v2 == v && i2 < i)) {
-    v = v2;
-    i = i2;
-  }
-}
-
-// T = float: the mixed cycle's inverse; T = double: the FP64 inverse, written
-// in place over the dense block M (every block reads its rows of M before the
-// first cluster barrier and writes them after the last one)
-template <class T, int NT>
-__global__ void __launch_bounds__(NT)
-k_gj_cluster(int na, int R, const double* M, T* out, int* __restrict__ flag) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ __align__(16) unsigned char gjc_raw[];
-  T* gjc_smem = reinterpret_cast<T*>(gjc_raw);
-  __shared__ T cand_v[2][kGjCluster];
-  __shared__ int cand_i[2][kGjCluster];
-  __shared__ T s_f[256];  // multipliers of the own rows (R <= 256)
-  __shared__ int s_p, s_src, s_cand, s_sing;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int CS = int(cluster.num_blocks());
-  const int rank = int(cluster.block_rank());
-  const int r0 = min(na, rank * R), r1 = min(na, r0 + R), nr = r1 - r0;
-  // column-major thread layout of the elimination: CW threads per row pass
-  const int na32 = (na + 31) & ~31;
-  const int G = max(1, NT / na32), CW = NT / G;
-  const int tx = t % CW, ty = t / CW;
-  T* own = gjc_smem;                    // [R][na]
-  T* pubrow = own + (size_t)R * na;     // [2][na] pivot candidate for the next column
-  T* oldrow = pubrow + 2 * (size_t)na;  // [2][na] the row at the next position (pushed by its owner)
-  T* prow = oldrow + 2 * (size_t)na;    // scaled pivot row of the step
-  int* perm_s = reinterpret_cast<int*>(prow + na);  // pivot positions
-  for (int e = t; e < nr * na; e += NT) own[e] = T(M[(size_t)r0 * na + e]);
-  if (t == 0) s_sing = 0;
-  __syncthreads();
-  auto publish = [&](int col, int buf) {
-    if (warp == 0) {
-      T v = -T(1.0);
-      int i = na;
-      for (int q = lane; q < nr; q += 32)
-        if (r0 + q >= col) gj_merge<T>(v, i, fabs(own[(size_t)q * na + col]), r0 + q);
+  for (int s = 0; s < RPT; ++s) {
+    const int r = k0 + t + s * bd;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const T v2 = __shfl_xor_sync(0xffffffffu, v, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        gj_merge<T>(v, i, v2, i2);
+    for (int j = 0; j < NB; ++j) row[s][j] = (r < n && j < nb) ? M[(size_t)r * n + k0 + j] : T(0);
+  }
+  for (int r = t; r < n; r += bd) sp[r] = r;
+  // The columns rotate by one place per step, so that the step's column is
+  // always row[s][0] and the loop body stays rolled (unrolled over the steps, the
+  // panel took 2 us per column fetching instructions); NB rotations put them back.
+#pragma unroll 1
+  for (int k = 0; k < NB; ++k) {
+    if (k >= nb) {  // uniform: the last panel's missing columns
+#pragma unroll
+      for (int s = 0; s < RPT; ++s) {
+        const T first = row[s][0];
+#pragma unroll
+        for (int j = 1; j < NB; ++j) row[s][j - 1] = row[s][j];
+        row[s][NB - 1] = first;
       }
-      if (lane < CS) {  // into every block's candidate table
-        cluster.map_shared_rank(&cand_v[buf][0], lane)[rank] = v;
-        cluster.map_shared_rank(&cand_i[buf][0], lane)[rank] = i;
-      }
-      if (lane == 0) s_cand = i < na ? i - r0 : -1;
+      continue;
     }
-    __syncthreads();
-    if (s_cand >= 0)
-      for (int j = t; j < na; j += NT) pubrow[(size_t)buf * na + j] = own[(size_t)s_cand * na + j];
-    if (col >= r0 && col < r1)  // the old row of the next step, into every block
-      for (int q = 0; q < CS; ++q) {
-        T* dst = cluster.map_shared_rank(oldrow, q) + (size_t)buf * na;
-        for (int j = t; j < na; j += NT) dst[j] = own[(size_t)(col - r0) * na + j];
+    const int kk = k0 + k, buf = k & 1;
+    unsigned long long key = 0;
+    int p = n;
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int r = k0 + t + s * bd;
+      const unsigned long long a = gj_key(row[s][0]);
+      if (r >= kk && r < n && (a > key || p == n)) {  // rows in increasing order: ties keep the smaller
+        key = a;
+        p = r;
       }
-  };
-  publish(0, 0);
-  cluster.sync();
-  for (int k = 0; k < na; ++k) {
-    const int buf = k & 1;
-    if (warp == 0) {  // the pivot: the same reduction in every block
-      T v = -T(1.0);
-      int i = na;
-      if (lane < CS) {
-        v = cand_v[buf][lane];
-        i = cand_i[buf][lane];
+    }
+    gj_warp_best<WIDE>(key, p, n);
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int r = k0 + t + s * bd;
+      if (r == p) {
+        wkey[buf][warp] = key;
+        wpos[buf][warp] = p;
+#pragma unroll
+        for (int j = 0; j < NB; ++j) cand[buf][warp][j] = row[s][j];
+      }
+      if (r == kk)
+#pragma unroll
+        for (int j = 0; j < NB; ++j) orow[buf][j] = row[s][j];
+    }
+    if (p == n && lane == 0) {  // no candidate in this warp
+      wkey[buf][warp] = 0;
+      wpos[buf][warp] = n;
+    }
+    // one barrier per step: the buffers of step k are written again at step
+    // k + 2, after the barrier of step k + 1, which every thread reaches only
+    // when it has read them
+    __syncthreads();
+    key = lane < nw ? wkey[buf][lane] : 0;
+    p = lane < nw ? wpos[buf][lane] : n;
+    gj_warp_best<WIDE>(key, p, n);
+    const bool singular = key == 0;
+    if (singular) p = kk;
+    const T* pr = singular ? orow[buf] : cand[buf][((p - k0) % bd) >> 5];
+    const T rpv = T(1) / (singular ? T(1) : pr[0]);
+    // the step for the other rows: the pivot row, its reciprocal on the diagonal
+    if (t < NB) steps[k * NB + (k + t) % NB] = t == 0 ? rpv : pr[t];
+    if (t == 0) {
+      const int a = sp[kk];
+      sp[kk] = sp[p];
+      sp[p] = a;
+      if (singular) *flag = 1;
+    }
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int r = k0 + t + s * bd;
+      if (r == p && p != kk)  // the displaced row moves here
+#pragma unroll
+        for (int j = 0; j < NB; ++j) row[s][j] = orow[buf][j];
+      // the pivot row becomes 0 + rpv (pivot row), column k of every row -g
+      T g = row[s][0] * rpv;
+      if (r == kk) {
+        g = -rpv;
+#pragma unroll
+        for (int j = 1; j < NB; ++j) row[s][j] = T(0);
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const T v2 = __shfl_xor_sync(0xffffffffu, v, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        gj_merge<T>(v, i, v2, i2);
-      }
-      if (lane == 0) {
-        const bool singular = !(v > T(0.0));
-        s_p = singular ? k : i;
-        s_src = singular ? -1 : i / R;  // -1: the pivot row is the old row k
-        perm_s[k] = s_p;
-        if (singular) s_sing = 1;
-      }
-    }
-    __syncthreads();
-    const int p = s_p;
-    const T* old = oldrow + (size_t)buf * na;
-    const T* src = s_src < 0 ? old : cluster.map_shared_rank(pubrow, s_src) + (size_t)buf * na;
-    const T pv = s_src < 0 ? T(1.0) : src[k];
-    for (int j = t; j < na; j += NT) prow[j] = (j == k ? T(1.0) : src[j]) / pv;
-    if (t < nr) {
-      const int i = r0 + t;
-      s_f[t] = (i == p && p != k) ? old[k] : own[(size_t)t * na + k];
-    }
-    __syncthreads();
-    for (int j = tx; j < na; j += CW) {
-      const T pj = prow[j], oj = old[j];
-      const bool jk = j == k;
-      for (int ii = ty; ii < nr; ii += G) {  // the row index is the same across a warp
-        const int i = r0 + ii;
-        T* Mij = own + (size_t)ii * na + j;
-        if (i != k && i != p) {
-          *Mij = (jk ? T(0.0) : *Mij) - s_f[ii] * pj;
-        } else if (i == k) {
-          *Mij = pj;
-        } else {  // i == p != k: the old row k moves here
-          *Mij = (jk ? T(0.0) : oj) - s_f[ii] * pj;
-        }
-      }
-    }
-    __syncthreads();
-    if (k + 1 < na) publish(k + 1, buf ^ 1);
-    cluster.sync();  // publications visible; every block is done reading this step's
-  }
-  // undo the column swaps (k_gj_unswap) on the own rows, write them out
-  for (int q = t; q < nr; q += NT) {
-    T* row = own + (size_t)q * na;
-    for (int k = na - 1; k >= 0; --k) {
-      const int pk = perm_s[k];
-      if (pk != k) {
-        const T a = row[k];
-        row[k] = row[pk];
-        row[pk] = a;
-      }
+      for (int j = 1; j < NB; ++j) row[s][j - 1] = row[s][j] - g * pr[j];
+      row[s][NB - 1] = -g;
     }
   }
   __syncthreads();
-  for (int e = t; e < nr * na; e += NT) out[(size_t)r0 * na + e] = own[e];
-  if (t == 0 && s_sing) *flag = 1;
+  if (t < nb)  // positions k0 .. k0 + nb - 1 belong to the first threads
+#pragma unroll
+    for (int j = 0; j < NB; ++j) D[t * NB + j] = j < nb ? row[0][j] : T(0);
+  // the swaps touch positions from k0 on; every thread reads its old entries
+  // before the barrier and writes after it
+  int from[RPT];
+#pragma unroll
+  for (int s = 0; s < RPT; ++s) {
+    const int r = k0 + t + s * bd;
+    from[s] = r >= n ? 0 : k0 == 0 ? sp[r] : rowsrc[sp[r]];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < RPT; ++s)
+    if (k0 + t + s * bd < n) rowsrc[k0 + t + s * bd] = from[s];
+  for (int r = t; r < n; r += bd) prm[r] = sp[r];
+}
+
+// TR x 32 tile per block of 32 x 8 threads; cols: the last panel's column map
+template <class T, int NB, int TR>
+__global__ void __launch_bounds__(256) k_gj_apply(int n, int k0, int nb, const T* __restrict__ src,
+                                                  const T* __restrict__ D, const T* __restrict__ steps,
+                                                  const int* __restrict__ prm, const int* __restrict__ cols,
+                                                  T* __restrict__ dst) {
+  constexpr int QR = TR / 8;
+  static_assert(256 % NB == 0 && NB <= 32 && (TR * NB) % 32 == 0, "one thread per panel entry, rows within a warp");
+  __shared__ T w[TR][NB + 1], piv[NB][32], st[NB][NB];
+  const int tx = threadIdx.x, ty = threadIdx.y, t = ty * 32 + tx;
+  const int i0 = blockIdx.y * TR, j = blockIdx.x * 32 + tx;
+  pdl_enter();
+  for (int e = t; e < NB * NB; e += 256) st[e / NB][e % NB] = e / NB < nb ? steps[e] : T(0);
+  for (int l = ty; l < NB; l += 8) piv[l][tx] = (l < nb && j < n) ? src[(size_t)prm[k0 + l] * n + j] : T(0);
+  T acc[QR];
+#pragma unroll
+  for (int q = 0; q < QR; ++q) {
+    const int i = i0 + ty + 8 * q;
+    acc[q] = (i < n && j < n && (i < k0 || i >= k0 + nb)) ? src[(size_t)prm[i] * n + j] : T(0);
+  }
+  __syncthreads();
+  // the panel's steps on the tile's rows, one thread per entry; the panel's own
+  // rows come from k_gj_panel
+  for (int e = t; e < TR * NB; e += 256) {
+    const int r = e / NB, l = e % NB, i = i0 + r;
+    T v = (i < n && l < nb) ? src[(size_t)prm[i] * n + k0 + l] : T(0);
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+      const T g = __shfl_sync(0xffffffffu, v, k, NB) * st[k][k];
+      if (k < nb) v = l == k ? -g : v - g * st[k][l];
+    }
+    w[r][l] = (i >= k0 && i < k0 + nb) ? D[(i - k0) * NB + l] : v;
+  }
+  __syncthreads();
+  if (j >= n) return;
+  const bool own = j >= k0 && j < k0 + nb;  // a column of the panel
+  const int jo = cols ? cols[j] : j;
+#pragma unroll
+  for (int q = 0; q < QR; ++q) {
+    const int r = ty + 8 * q, i = i0 + r;
+    if (i >= n) continue;
+    T s = acc[q];
+    if (own) {
+      s = w[r][j - k0];
+    } else {
+#pragma unroll
+      for (int l = 0; l < NB; ++l) s += w[r][l] * piv[l][tx];
+    }
+    dst[(size_t)i * n + jo] = s;
+  }
+}
+
+// launch with programmatic stream serialization: the kernel begins with
+// pdl_enter()
+template <class... KArgs, class... Args>
+static void launch_pdl(pm_ctx* c, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c->pdl >= 1 ? 1 : 0;
+  PM_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+  c->kernel_launches++;
+}
+
+template <class T, int NB, int RPT, int TR>
+static void gj_panels(pm_ctx* c, int n, T* a, T* b, T* d, int* prm, int* rowsrc, int* flag, T* out) {
+  const dim3 grid((n + 31) / 32, (n + TR - 1) / TR), block(32, 8);
+  const size_t smem = size_t(n) * sizeof(int);
+  for (int k0 = 0; k0 < n; k0 += NB) {
+    const int nb = std::min(NB, n - k0), rows = n - k0;
+    const bool last = k0 + nb == n;
+    if (rows <= 1024)
+      launch_pdl(c, k_gj_panel<T, NB, 1>, dim3(1), dim3((rows + 31) & ~31), smem, n, k0, nb, a, d, d + NB * NB, prm, rowsrc,
+                 flag);
+    else if (RPT > 1 && rows <= 2048)
+      launch_pdl(c, k_gj_panel<T, NB, (RPT > 1 ? RPT / 2 : 1)>, dim3(1), dim3(1024), smem, n, k0, nb, a, d, d + NB * NB, prm, rowsrc,
+                 flag);
+    else
+      launch_pdl(c, k_gj_panel<T, NB, RPT>, dim3(1), dim3(1024), smem, n, k0, nb, a, d, d + NB * NB, prm, rowsrc,
+                 flag);
+    launch_pdl(c, k_gj_apply<T, NB, TR>, grid, block, 0, n, k0, nb, a, d, d + NB * NB, prm,
+               last ? rowsrc : nullptr, last ? out : b);
+    std::swap(a, b);
+  }
+}
+
+// Panel widths, by the same update: FP64 343 rows 910 / 822 / 962 us with 4 / 8 /
+// 16 columns (a step's FP64 work grows with the width, the launches fall with
+// it); FP32 469 / 416 / 459 us with 8 / 16 / 32 (with W formed from D).
+static void gj_inverse(pm_ctx* c, int n, float* a, float* b, float* d, int* prm, int* rowsrc, int* flag, float* out) {
+  gj_panels<float, 16, 1, 16>(c, n, a, b, d, prm, rowsrc, flag, out);
+}
+static void gj_inverse(pm_ctx* c, int n, double* a, double* b, double* d, int* prm, int* rowsrc, int* flag,
+                       double* out) {
+  gj_panels<double, 8, 4, 16>(c, n, a, b, d, prm, rowsrc, flag, out);
 }
 
 __global__ void k_coarse_gemv32(int n, int na, const int* __restrict__ act, const int* __restrict__ pos,
@@ -1348,6 +1341,14 @@ __global__ void k_coarse_gemv_mixed(int n, int na, const int* __restrict__ act, 
   }
 }
 
+// launches go to another stream for the lifetime of the object
+struct StreamSwap {
+  pm_ctx* c;
+  cudaStream_t saved;
+  StreamSwap(pm_ctx* c_, cudaStream_t s_) : c(c_), saved(c_->stream) { c->stream = s_; }
+  ~StreamSwap() { c->stream = saved; }
+};
+
 void DenseInverse::solve_mixed(pm_ctx* c, const float* b, float* x) {
   if (!has64) throw Error(PM_E_INVALID, "coarse solve before the FP64 inverse was built");
   const long long threads = (long long)na * 32 + n;
@@ -1360,24 +1361,15 @@ void DenseInverse::build32(pm_ctx* c, const DevCsr& A) {
   complete32(c, A);
 }
 
+// the active rows that the FP32 inverse is computed for in FP32; larger ones
+// take the FP64 inverse, rounded
+constexpr int kGjRows32 = 640;
+
 void DenseInverse::launch32(pm_ctx* c, const DevCsr& A, cudaStream_t s) {
   pending32 = false;
-  n = A.n_rows;
-  int na_ = 0;
-  for (int i = 0; i < n; ++i)
-    for (int b = 0; b < A.mask.nb; ++b)
-      if (i >= A.mask.start[b] && i < A.mask.end[b] && i < A.mask.active_end[b]) ++na_;
-  // one block when the whole active block fits its shared memory, else a
-  // cluster of kGjCluster blocks
-  auto smem_for = [&](int R) { return (size_t(R) + 5) * na_ * sizeof(float) + size_t(na_) * sizeof(int); };
-  int cs = std::max(1, std::min(kGjCluster, c->coarse_cluster)), R = (na_ + cs - 1) / cs;
-  while (cs < kGjCluster && smem_for(R) > kGjClusterSmem) {
-    cs *= 2;
-    R = (na_ + cs - 1) / cs;
-  }
-  const size_t smem = smem_for(R);
-  if (na_ == 0 || R > 256 || smem > kGjClusterSmem) {
-    build(c, A);  // large: the FP64 inverse, rounded
+  set_rows(c, A);
+  if (na == 0 || na > kGjRows32) {
+    build(c, A);
     inv32.ensure(size_t(na) * na);
     if (na) {
       k_d2f<<<grid_for(c, (long long)na * na), 256, 0, c->stream>>>((long long)na * na, inv.p, inv32.p);
@@ -1387,50 +1379,13 @@ void DenseInverse::launch32(pm_ctx* c, const DevCsr& A, cudaStream_t s) {
     has32 = true;
     return;
   }
-  // the preparation and the kernel on stream s (restored on every exit)
-  struct StreamSwap {
-    pm_ctx* c;
-    cudaStream_t saved;
-    StreamSwap(pm_ctx* c_, cudaStream_t s_) : c(c_), saved(c_->stream) { c->stream = s_; }
-    ~StreamSwap() { c->stream = saved; }
-  } swap(c, s);
-  prepare(c, A);  // act, pos, the dense active block in inv (FP64)
-  inv32.ensure(size_t(na) * na);
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(k_gj_cluster<float, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(kGjClusterSmem));
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(k_gj_cluster<float, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(kGjClusterSmem));
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(k_gj_cluster<float, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(kGjClusterSmem));
-  });
-  PM_CUDA(attr_err);
-  // measured on GB300 (225 and 343 active rows): 8 blocks of 1024 threads
-  const int nt = c->coarse_threads > 0 ? c->coarse_threads : 1024;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(cs));
-  cfg.blockDim = dim3(unsigned(nt));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = unsigned(cs);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const double* Mp = inv.p;
-  float* outp = inv32.p;
-  int* fl = flag.p;
-  int na_arg = na, R_arg = R;
-  if (nt == 1024) PM_CUDA(cudaLaunchKernelEx(&cfg, k_gj_cluster<float, 1024>, na_arg, R_arg, Mp, outp, fl));
-  else if (nt == 512) PM_CUDA(cudaLaunchKernelEx(&cfg, k_gj_cluster<float, 512>, na_arg, R_arg, Mp, outp, fl));
-  else PM_CUDA(cudaLaunchKernelEx(&cfg, k_gj_cluster<float, 256>, na_arg, R_arg, Mp, outp, fl));
-  c->kernel_launches++;
+  // the preparation and the kernels on stream s (restored on every exit)
+  StreamSwap swap(c, s);
+  const size_t nn = size_t(na) * na;
+  inv32.ensure(nn);
+  work32.ensure(2 * nn + 2 * 16 * 16);
+  prepare(c, A, work32.p);
+  gj_inverse(c, na, work32.p, work32.p + nn, work32.p + 2 * nn, perm.p, perm.p + na, flag.p, inv32.p);
   if (!done_event) PM_CUDA(cudaEventCreateWithFlags(&done_event, cudaEventDisableTiming));
   PM_CUDA(cudaEventRecord(done_event, s));
   pending32 = true;
@@ -1455,7 +1410,6 @@ void DenseInverse::complete32(pm_ctx* c, const DevCsr& A) {
     has32 = true;
     return;
   }
-  has64 = false;  // inv holds the active block, not its inverse
   has32 = true;
 }
 
@@ -1466,7 +1420,14 @@ void DenseInverse::solve32(pm_ctx* c, const float* b, float* x) {
              (const int*)pos.p, (const float*)inv32.p, b, x);
 }
 
-void DenseInverse::prepare(pm_ctx* c, const DevCsr& A) {
+// the active rows depend on the block layout only; kept until it changes
+void DenseInverse::set_rows(pm_ctx* c, const DevCsr& A) {
+  bool same = act_set && n == A.n_rows && rows_of.nb == A.mask.nb;
+  for (int b = 0; same && b < A.mask.nb; ++b)
+    same = rows_of.start[b] == A.mask.start[b] && rows_of.active_end[b] == A.mask.active_end[b] &&
+           rows_of.end[b] == A.mask.end[b];
+  if (same) return;
+  act_set = false;
   n = A.n_rows;
   std::vector<int> h_act, h_pos(n, -1);
   for (int i = 0; i < n; ++i) {
@@ -1482,15 +1443,22 @@ void DenseInverse::prepare(pm_ctx* c, const DevCsr& A) {
   if (na > 20000) throw Error(PM_E_UNSUPPORTED, "coarse direct solve limited to 20000 active rows");
   act.upload(h_act, c->stream);
   pos.upload(h_pos, c->stream);
-  inv.ensure(size_t(na) * na);
   tmp.ensure(std::max(na, 1));
-  perm.ensure(std::max(na, 1));
+  perm.ensure(2 * std::max(na, 1));
   flag.ensure(1);
+  PM_CUDA(cudaStreamSynchronize(c->stream));  // the host vectors go out of scope
+  rows_of = A.mask;
+  rows_of.guard = nullptr;
+  act_set = true;
+}
+
+template <class T>
+void DenseInverse::prepare(pm_ctx* c, const DevCsr& A, T* M) {
   PM_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), c->stream));
   has64 = has32 = false;
   if (na == 0) return;
-  k_dense_fill<<<nblocks(na, 128), 128, 0, c->stream>>>(na, act.p, pos.p, A.row_ptr.p, A.cols.p,
-                                                        A.vals.p, inv.p);
+  k_dense_fill<T><<<nblocks((long long)na * 32, 256), 256, 0, c->stream>>>(na, act.p, pos.p, A.row_ptr.p, A.cols.p,
+                                                                         A.vals.p, M);
   PM_CHECK_LAUNCH();
   c->kernel_launches++;
 }
@@ -1513,102 +1481,35 @@ void DenseInverse::complete64(pm_ctx* c) {
 
 void DenseInverse::launch64(pm_ctx* c, const DevCsr& A, cudaStream_t s) {
   pending64 = false;
-  struct StreamSwap {
-    pm_ctx* c;
-    cudaStream_t saved;
-    StreamSwap(pm_ctx* c_, cudaStream_t s_) : c(c_), saved(c_->stream) { c->stream = s_; }
-    ~StreamSwap() { c->stream = saved; }
-  } swap(c, s);
-  prepare(c, A);
-  if (na == 0) {
-    has64 = true;
-    return;
-  }
-  // Gauss-Jordan on one thread-block cluster when the active block fits its
-  // distributed shared memory (cluster barriers per column instead of grid
-  // barriers; the same pivot rule), in place
-  {
-    auto smem_for = [&](int R) { return (size_t(R) + 5) * na * sizeof(double) + size_t(na) * sizeof(int); };
-    int cs = std::max(1, std::min(kGjCluster, c->coarse_cluster)), R = (na + cs - 1) / cs;
-    while (cs < kGjCluster && smem_for(R) > kGjClusterSmem) {
-      cs *= 2;
-      R = (na + cs - 1) / cs;
-    }
-    const size_t smem = smem_for(R);
-    if (R <= 256 && smem <= kGjClusterSmem) {
-      static std::once_flag once;
-      static cudaError_t attr_err = cudaSuccess;
-      std::call_once(once, [] {
-        attr_err = cudaFuncSetAttribute(k_gj_cluster<double, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(kGjClusterSmem));
-        if (attr_err == cudaSuccess)
-          attr_err = cudaFuncSetAttribute(k_gj_cluster<double, 512>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGjClusterSmem));
-        if (attr_err == cudaSuccess)
-          attr_err = cudaFuncSetAttribute(k_gj_cluster<double, 256>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGjClusterSmem));
-      });
-      PM_CUDA(attr_err);
-      const int nt = c->coarse_threads > 0 ? c->coarse_threads : 1024;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(unsigned(cs));
-      cfg.blockDim = dim3(unsigned(nt));
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = s;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = unsigned(cs);
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      const double* Mp = inv.p;
-      double* outp = inv.p;
-      int* fl = flag.p;
-      int na_arg = na, R_arg = R;
-      if (nt == 1024) PM_CUDA(cudaLaunchKernelEx(&cfg, k_gj_cluster<double, 1024>, na_arg, R_arg, Mp, outp, fl));
-      else if (nt == 512) PM_CUDA(cudaLaunchKernelEx(&cfg, k_gj_cluster<double, 512>, na_arg, R_arg, Mp, outp, fl));
-      else PM_CUDA(cudaLaunchKernelEx(&cfg, k_gj_cluster<double, 256>, na_arg, R_arg, Mp, outp, fl));
-      c->kernel_launches++;
-      if (!done_event) PM_CUDA(cudaEventCreateWithFlags(&done_event, cudaEventDisableTiming));
-      PM_CUDA(cudaEventRecord(done_event, s));
-      pending64 = true;
+  set_rows(c, A);
+  StreamSwap swap(c, s);
+  const size_t nn = size_t(na) * na;
+  inv.ensure(nn);
+  const bool panels = na <= kGjMaxRows;
+  if (panels && na) {
+    work.ensure(2 * nn + 2 * 8 * 8);
+    prepare(c, A, work.p);
+    gj_inverse(c, na, work.p, work.p + nn, work.p + 2 * nn, perm.p, perm.p + na, flag.p, inv.p);
+  } else {
+    prepare(c, A, inv.p);
+    if (na == 0) {
+      has64 = true;
       return;
     }
+    eliminate_columns(c);
   }
+  if (!done_event) PM_CUDA(cudaEventCreateWithFlags(&done_event, cudaEventDisableTiming));
+  PM_CUDA(cudaEventRecord(done_event, s));
+  pending64 = true;
+}
+
+// Column by column, in place: more rows than the panel's block keeps in
+// registers
+void DenseInverse::eliminate_columns(pm_ctx* c) {
   int coop = 0, per_sm = 0;
   PM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
   PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gj_coop, 256, 0));
-  // row-resident variant: R rows per block (at most 32), rows and two row
-  // buffers in shared memory
-  const int R = std::max(2, (na + c->num_sms - 1) / c->num_sms);
-  const size_t rsmem = size_t(R + 2) * na * sizeof(double);
-  const int rblocks = (na + R - 1) / R;
-  int rows_per_sm = 0;
-  if (coop && R <= 32 && rsmem <= kGjRowsSmem) {
-    static std::once_flag once;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(once, [] {
-      attr_err = cudaFuncSetAttribute(k_gj_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGjRowsSmem));
-    });
-    PM_CUDA(attr_err);
-    PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rows_per_sm, k_gj_rows, 256, rsmem));
-  }
-  if (rows_per_sm > 0 && rows_per_sm * c->num_sms >= rblocks) {
-    pub_rows.ensure(2 * size_t(rblocks + 1) * na);
-    pub_v.ensure(2 * size_t(rblocks));
-    pub_i.ensure(2 * size_t(rblocks));
-    double* M = inv.p;
-    int* pp = perm.p;
-    double* pr = pub_rows.p;
-    double* pv = pub_v.p;
-    int* pi = pub_i.p;
-    int* fl = flag.p;
-    int nan_ = na, R_ = R;
-    void* args[] = {&nan_, &R_, &M, &pp, &pr, &pv, &pi, &fl};
-    PM_CUDA(cudaLaunchCooperativeKernel((const void*)k_gj_rows, dim3(rblocks), dim3(256), args, rsmem, c->stream));
-    c->kernel_launches++;
-  } else if (coop && per_sm > 0) {
+  if (coop && per_sm > 0) {
     // one cooperative launch; at most one block per SM and about 8 rows per block
     int nb = std::min(c->num_sms, std::max(1, (na + 7) / 8));
     rowk.ensure(na);
@@ -1639,9 +1540,6 @@ void DenseInverse::launch64(pm_ctx* c, const DevCsr& A, cudaStream_t s) {
   k_gj_unswap<<<nblocks(na, 128), 128, 0, c->stream>>>(na, inv.p, perm.p);
   PM_CHECK_LAUNCH();
   c->kernel_launches++;
-  if (!done_event) PM_CUDA(cudaEventCreateWithFlags(&done_event, cudaEventDisableTiming));
-  PM_CUDA(cudaEventRecord(done_event, s));
-  pending64 = true;
 }
 
 // tmp_a = b_a - sum over non-active columns of A_{a,j} b_j

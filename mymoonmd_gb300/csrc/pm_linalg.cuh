@@ -146,25 +146,27 @@ struct DenseInverse {
   DBuf<int> act;     // active row indices (na)
   DBuf<int> pos;     // row -> position among the active rows, -1 if non-active
   DBuf<double> tmp;  // na
-  DBuf<int> perm;    // pivot rows (na)
+  DBuf<int> perm;    // pivot rows (na), composed row swaps (na)
   DBuf<int> flag;    // singular pivot flag
-  DBuf<double> rowk, oldk, part_v;  // cooperative elimination: pivot row, old row k, block arg-max
+  DBuf<double> rowk, oldk, part_v;  // column-by-column elimination: pivot row, old row k, block arg-max
   DBuf<int> part_i;
-  // row-resident elimination: per step, every block's candidate pivot row and
-  // the old row k, double-buffered ([2][blocks + 1][na]), and the candidates'
-  // arg-max values and positions ([2][blocks])
-  DBuf<double> pub_rows, pub_v;
-  DBuf<int> pub_i;
+  // blocked elimination: the matrix before and after a panel, the panel
+  DBuf<double> work;
+  DBuf<float> work32;
+  BlockMask rows_of{};   // the block layout act / pos were made for
+  bool act_set = false;
   // FP32 inverse for the mixed-precision cycle (build32); has64/has32: which
   // inverse holds the current matrix
   DBuf<float> inv32;
   bool has64 = false, has32 = false;
   void build(pm_ctx* c, const DevCsr& A);
-  // act, pos and the dense active block (FP64) in inv
-  void prepare(pm_ctx* c, const DevCsr& A);
-  // the FP32 inverse: Gauss-Jordan in FP32 on one thread-block cluster when
-  // the active block fits its distributed shared memory, else the FP64
-  // inverse rounded to FP32
+  void set_rows(pm_ctx* c, const DevCsr& A);  // n, na, act, pos
+  // the dense active block into M, the pivot flag cleared
+  template <class T>
+  void prepare(pm_ctx* c, const DevCsr& A, T* M);
+  void eliminate_columns(pm_ctx* c);  // inv := inv^-1, column by column
+  // the FP32 inverse: Gauss-Jordan in FP32 for up to 640 active rows, else the
+  // FP64 inverse rounded to FP32
   void build32(pm_ctx* c, const DevCsr& A);
   // build32 in two halves: launch32 queues the factorisation on the stream s
   // (no host synchronisation; the large-matrix path runs build() at once),
