@@ -14,6 +14,8 @@
 // VankaSmoother::smooth (src/Multigrid/VankaSmoother.C:110-292).
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -993,6 +995,166 @@ void DevNodalVanka::build_row_slices(pm_ctx* c, const pmsetup::Csr& S, int p0, c
   rs_ok = true;
 }
 
+// The share of one warp in the residual of a patch: 8 rows, steps [a0, a0 + na)
+// of A and [b0, b0 + nb) of B^T, the partial sum's slot
+struct NodalChunk {
+  unsigned short a0, b0;
+  unsigned char na, nb, part, pad;
+};
+static_assert(sizeof(NodalChunk) == sizeof(uint2), "one 8-byte load");
+constexpr size_t kNodalPatchSmem = 200 * 1024;  // of the 227 KB a block may have, its static part aside
+// A steps per chunk (a long row's steps go to several warps) and partial sums
+// per row
+constexpr int kNodalSteps = 9, kNodalParts = 3;
+
+// The patches packed for k_nodal_patch. False if they do not fit it: more than
+// 32 colours (the mask's bits), longer rows than kNodalParts chunks, velocity
+// components that couple or differ.
+bool DevNodalVanka::build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vector<int>& vp,
+                               const std::vector<int>& vi, const std::vector<int>& color, int n_colors) {
+  if (n_colors > 32 || max_nodes > kNodalMaxNodes) return false;
+  constexpr int C = 8, Lanes = 4;
+  std::vector<int> voff(size_t(np) + 1, 0), ioff(size_t(np) + 1, 0), ch0(size_t(np) + 1, 0), hptr(size_t(np) + 1, 0),
+      hnv(np), halo, src;
+  std::vector<uint2> chunks;
+  std::vector<unsigned char> row;
+  std::vector<unsigned short> idx;
+  std::vector<unsigned> mask(size_t(nu) + np, 0u);
+  std::vector<int> at(size_t(nu), -1), atp(size_t(np), -1), order, len, lenp, hp, sa, sb;
+  int64_t nv32 = 0, ni32 = 0;
+  pk_smem32.assign(size_t(n_colors) + 1, 0);
+  pk_smem64.assign(size_t(n_colors) + 1, 0);
+  for (int i = 0; i < np; ++i) {
+    const int m = vp[i + 1] - vp[i];
+    const int* nd = vi.data() + vp[i];
+    mask[size_t(nu) + i] |= 1u << color[i];
+    // halo: the patch's own nodes first, in order, then the nodes and pressures
+    // their rows couple to
+    const size_t h0 = halo.size();
+    int nh = 0;
+    hp.clear();
+    for (int a = 0; a < m; ++a) {
+      mask[size_t(nd[a])] |= 1u << color[i];
+      at[size_t(nd[a])] = nh++;
+      halo.push_back(nd[a]);
+    }
+    len.assign(m, 0);
+    lenp.assign(m, 0);
+    for (int a = 0; a < m; ++a) {
+      const int r0 = S.row_ptr[nd[a]], r1 = S.row_ptr[nd[a] + 1];
+      for (int k = 1; k < 3; ++k)
+        if (S.row_ptr[k * nu + nd[a] + 1] - S.row_ptr[k * nu + nd[a]] != r1 - r0) return false;
+      for (int k = r0; k < r1; ++k) {
+        const int col = S.cols[k];
+        if (col < nu) {
+          ++len[a];
+          if (at[size_t(col)] < 0) {
+            at[size_t(col)] = nh++;
+            halo.push_back(col);
+          }
+        } else if (col >= 3 * nu) {
+          ++lenp[a];
+          if (atp[size_t(col) - 3 * nu] < 0) {
+            atp[size_t(col) - 3 * nu] = int(hp.size());
+            hp.push_back(col - 3 * nu);
+          }
+        } else {
+          return false;  // the velocity components couple
+        }
+      }
+    }
+    if (nh + int(hp.size()) > 65535) return false;
+    halo.insert(halo.end(), hp.begin(), hp.end());
+    hnv[i] = nh;
+    hptr[size_t(i) + 1] = int(halo.size());
+    // slices of 8 rows, longest first
+    order.resize(m);
+    for (int a = 0; a < m; ++a) order[a] = a;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return len[a] > len[b]; });
+    const int nsl = (m + C - 1) / C;
+    sa.assign(size_t(nsl) + 1, 0);
+    sb.assign(size_t(nsl) + 1, 0);
+    for (int sl = 0; sl < nsl; ++sl) {
+      int ta = 0, tb_ = 0;
+      for (int q = 0; q < C && sl * C + q < m; ++q) {
+        ta = std::max(ta, (len[order[sl * C + q]] + Lanes - 1) / Lanes);
+        tb_ = std::max(tb_, (lenp[order[sl * C + q]] + Lanes - 1) / Lanes);
+      }
+      const int parts = std::max(1, (ta + kNodalSteps - 1) / kNodalSteps);
+      if (parts > kNodalParts) return false;
+      for (int k = 0; k < parts; ++k) {
+        const int a0 = ta * k / parts, a1 = ta * (k + 1) / parts;
+        NodalChunk ch{};
+        ch.a0 = (unsigned short)(sa[sl] + a0);
+        ch.na = (unsigned char)(a1 - a0);
+        ch.b0 = (unsigned short)sb[sl];
+        ch.nb = (unsigned char)(k == parts - 1 ? tb_ : 0);  // B^T with the last part
+        ch.part = (unsigned char)k;
+        uint2 raw;
+        std::memcpy(&raw, &ch, sizeof(raw));
+        chunks.push_back(raw);
+        for (int q = 0; q < C; ++q)
+          row.push_back(sl * C + q < m ? (unsigned char)order[sl * C + q] : (unsigned char)255);
+      }
+      sa[size_t(sl) + 1] = sa[sl] + ta;
+      sb[size_t(sl) + 1] = sb[sl] + tb_;
+    }
+    ch0[size_t(i) + 1] = int(chunks.size());
+    // values: the A steps of all slices, then the B^T steps (three components
+    // each); indices: A steps, B^T steps
+    const int na = sa[nsl], nb = sb[nsl];
+    const size_t v0 = src.size(), i0 = idx.size();
+    src.resize(v0 + size_t(32) * (size_t(na) + 3 * size_t(nb)), -1);
+    idx.resize(i0 + size_t(32) * (size_t(na) + nb), 0);
+    for (int sl = 0; sl < nsl; ++sl)
+      for (int q = 0; q < C && sl * C + q < m; ++q) {
+        const int a = order[sl * C + q], r0 = S.row_ptr[nd[a]];
+        int ja = 0, jb = 0;
+        for (int k = r0; k < S.row_ptr[nd[a] + 1]; ++k) {
+          const int col = S.cols[k];
+          if (col < nu) {
+            const size_t e = size_t(32) * (sa[sl] + ja / Lanes) + size_t(ja % Lanes) * C + q;
+            src[v0 + e] = k;
+            idx[i0 + e] = (unsigned short)at[size_t(col)];
+            ++ja;
+          } else {
+            const size_t step = size_t(sb[sl]) + jb / Lanes, lane = size_t(jb % Lanes) * C + q;
+            for (int d = 0; d < 3; ++d)
+              src[v0 + size_t(32) * (na + 3 * step + d) + lane] = S.row_ptr[d * nu + nd[a]] + (k - r0);
+            idx[i0 + size_t(32) * (na + step) + lane] = (unsigned short)atp[size_t(col) - 3 * nu];
+            ++jb;
+          }
+        }
+      }
+    nv32 += na + 3 * nb;
+    ni32 += na + nb;
+    for (int k : {color[i], n_colors}) {
+      const int inv = (m * m + 3) & ~3, rest = 32 * (na + 3 * nb) + 3 * nh + int(hp.size()), ix = 64 * (na + nb);
+      pk_smem32[k] = std::max(pk_smem32[k], 4 * (inv + rest) + ix);
+      pk_smem64[k] = std::max(pk_smem64[k], 8 * (inv + rest) + ix);
+    }
+    if (nv32 > 0x3ffffff) return false;  // entries stay below 2^31
+    voff[size_t(i) + 1] = int(nv32);
+    ioff[size_t(i) + 1] = int(ni32);
+    for (size_t t = h0; t < h0 + size_t(nh); ++t) at[size_t(halo[t])] = -1;
+    for (int v : hp) atp[size_t(v)] = -1;
+  }
+  pk_entries = 32 * nv32;
+  pk_voff.upload(voff, c->stream);
+  pk_ioff.upload(ioff, c->stream);
+  pk_chunk.upload(chunks, c->stream);
+  pk_ch0.upload(ch0, c->stream);
+  pk_hptr.upload(hptr, c->stream);
+  pk_hnv.upload(hnv, c->stream);
+  pk_row.upload(row, c->stream);
+  pk_idx.upload(idx, c->stream);
+  pk_halo_idx.upload(halo, c->stream);
+  pk_src.upload(src, c->stream);
+  pk_mask.upload(mask, c->stream);
+  PM_CUDA(cudaStreamSynchronize(c->stream));  // the host vectors go out of scope
+  return true;
+}
+
 // the periodic lattice colouring of the nodal patches (see setup); false if
 // the pressure nodes are not on a 3D lattice or two patches of one colour
 // share a velocity node
@@ -1049,7 +1211,7 @@ void DevNodalVanka::setup(pm_ctx* c, const DiscLevel& L) {
   for (int i = 0; i < np; ++i) {
     const int m = vp[i + 1] - vp[i];
     max_nodes = std::max(max_nodes, m);
-    ao[i + 1] = ao[i] + int64_t(m) * m;
+    ao[i + 1] = ao[i] + ((int64_t(m) * m + 3) & ~int64_t(3));  // 16-byte boundaries
   }
   if (max_nodes > kNodalMaxNodes)
     throw Error(PM_E_UNSUPPORTED, "nodal Vanka patch with " + std::to_string(max_nodes) +
@@ -1121,7 +1283,9 @@ void DevNodalVanka::setup(pm_ctx* c, const DiscLevel& L) {
     for (int i = 0; i < np; ++i) cp[fill[color[i]]++] = i;
   }
   color_patches.upload(cp, c->stream);
-  build_row_slices(c, S, L.pressure_row0, vp, vi, cp);
+  pk_ok = c->nodal_sliced == 8 && build_pack(c, S, vp, vi, color, n_colors) &&
+          size_t(std::max(pk_smem32.back(), pk_smem64.back())) <= kNodalPatchSmem;
+  if (!pk_ok) build_row_slices(c, S, L.pressure_row0, vp, vi, cp);
   color_entries.assign(n_colors, 0);
   color_rows.assign(n_colors, 0);
   color_nodes.assign(n_colors, 0);
@@ -1168,7 +1332,7 @@ __global__ void __launch_bounds__(256) k_nodal_factor(int np, int nu, const int*
                                                       const int* __restrict__ rp, const int* __restrict__ ci,
                                                       const T* __restrict__ v, T* __restrict__ ainv,
                                                       T* __restrict__ tb, T* __restrict__ sinv,
-                                                      int* __restrict__ flag) {
+                                                      T* __restrict__ cd, int* __restrict__ flag) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int i = blockIdx.x;
   if (i >= np) return;
@@ -1356,6 +1520,7 @@ __global__ void __launch_bounds__(256) k_nodal_factor(int np, int nu, const int*
     const T S = cdiag - s;
     if (!(S != T(0))) atomicExch(flag, 1);
     sinv[i] = S != T(0) ? T(1) / S : T(0);
+    cd[i] = cdiag;
   }
   T* out = ainv + aoff[i];
   for (int e = t; e < m * m; e += blockDim.x) {
@@ -1384,21 +1549,21 @@ static size_t nodal_factor_smem(int m) {
 
 template <class T, int TR>
 static void launch_nodal_factor_tr(pm_ctx* c, DevNodalVanka& nv, const int* rp, const int* ci, const T* v, T* ainv,
-                                   T* tb, T* sinv) {
+                                   T* tb, T* sinv, T* cd) {
   const size_t sm = nodal_factor_smem<T>(nv.max_nodes);
   PM_CUDA(cudaFuncSetAttribute(k_nodal_factor<T, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
   k_nodal_factor<T, TR><<<nv.np, 256, sm, c->stream>>>(nv.np, nv.nu, nv.vptr.p, nv.vidx.p, nv.aoff.p, rp, ci, v, ainv,
-                                                        tb, sinv, nv.flag.p);
+                                                        tb, sinv, cd, nv.flag.p);
 }
 
 // the register tile of the factor kernel covers 16 TR rows and columns
 template <class T>
 static void launch_nodal_factor(pm_ctx* c, DevNodalVanka& nv, const int* rp, const int* ci, const T* v, T* ainv,
-                                T* tb, T* sinv) {
+                                T* tb, T* sinv, T* cd) {
   static_assert(kNodalMaxNodes <= 96, "register tiles cover at most 96 nodes");
-  if (nv.max_nodes <= 64) launch_nodal_factor_tr<T, 4>(c, nv, rp, ci, v, ainv, tb, sinv);
-  else if (nv.max_nodes <= 80) launch_nodal_factor_tr<T, 5>(c, nv, rp, ci, v, ainv, tb, sinv);
-  else launch_nodal_factor_tr<T, 6>(c, nv, rp, ci, v, ainv, tb, sinv);
+  if (nv.max_nodes <= 64) launch_nodal_factor_tr<T, 4>(c, nv, rp, ci, v, ainv, tb, sinv, cd);
+  else if (nv.max_nodes <= 80) launch_nodal_factor_tr<T, 5>(c, nv, rp, ci, v, ainv, tb, sinv, cd);
+  else launch_nodal_factor_tr<T, 6>(c, nv, rp, ci, v, ainv, tb, sinv, cd);
 }
 
 void DevNodalVanka::factor(pm_ctx* c, const DevCsr& V, bool fp32) {
@@ -1407,17 +1572,33 @@ void DevNodalVanka::factor(pm_ctx* c, const DevCsr& V, bool fp32) {
     ainv32.ensure(size_t(ainv_len));
     tb32.ensure(size_t(6) * vidx.n);
     sinv32.ensure(np);
+    cdiag32.ensure(np);
     sol32.ensure(size_t(3) * vidx.n + np);
-    launch_nodal_factor<float>(c, *this, V.row_ptr.p, V.cols.p, V.vals32.p, ainv32.p, tb32.p, sinv32.p);
+    launch_nodal_factor<float>(c, *this, V.row_ptr.p, V.cols.p, V.vals32.p, ainv32.p, tb32.p, sinv32.p,
+                               cdiag32.p);
   } else {
     ainv.ensure(size_t(ainv_len));
     tb.ensure(size_t(6) * vidx.n);
     sinv.ensure(np);
+    cdiag.ensure(np);
     sol.ensure(size_t(3) * vidx.n + np);
-    launch_nodal_factor<double>(c, *this, V.row_ptr.p, V.cols.p, V.vals.p, ainv.p, tb.p, sinv.p);
+    launch_nodal_factor<double>(c, *this, V.row_ptr.p, V.cols.p, V.vals.p, ainv.p, tb.p, sinv.p, cdiag.p);
   }
   PM_CHECK_LAUNCH();
   c->kernel_launches++;
+  if (pk_ok) {
+    // the packed rows take the projected matrix's values (FP32: rounded FP64)
+    const int g = int(std::max<int64_t>(1, std::min<int64_t>((pk_entries + 255) / 256, int64_t(c->num_sms) * 8)));
+    if (fp32) {
+      pk_vals32.ensure(size_t(pk_entries));
+      k_fill_rows<float><<<g, 256, 0, c->stream>>>(pk_entries, pk_src.p, V.vals.p, pk_vals32.p);
+    } else {
+      pk_vals.ensure(size_t(pk_entries));
+      k_fill_rows<double><<<g, 256, 0, c->stream>>>(pk_entries, pk_src.p, V.vals.p, pk_vals.p);
+    }
+    PM_CHECK_LAUNCH();
+    c->kernel_launches++;
+  }
   if (rs_ok) {
     // the sliced rows take the projected matrix's values (FP32: rounded FP64)
     const int g = int(std::max<int64_t>(1, std::min<int64_t>((rs_entries + 255) / 256, int64_t(c->num_sms) * 8)));
@@ -1632,17 +1813,389 @@ __global__ void __launch_bounds__(512) k_nodal_rhs(const int* __restrict__ guard
   }
 }
 
+// One patch of a nodal Vanka sweep per block: its residual, its local solve and
+// its update in one kernel, one launch per colour.
+//
+// The patch comes packed: the rows of its m velocity nodes as sliced-ELL steps (8
+// rows, 4 lanes each, longest rows first) of the velocity block A, stored once
+// for the three components, and of the three B^T columns, with 16-bit indices
+// into the patch's halo (the nodes and pressures the rows couple to). The block
+// gathers the halo of x into shared memory, a warp sums a chunk of at most
+// kNodalSteps steps for all three components, and the Schur complement solve
+// follows as in k_nodal_local (r_p = b_p - b . u - c p comes with its dot
+// product).
+//
+// Within a colour every residual has to see the iterate before the colour's
+// updates, and patches of one colour read each other's nodes: the iterate goes
+// from xs to xd. xd already holds xs as of one colour before, so besides its own
+// nodes a block moves the nodes of one patch of the previous colour that this
+// colour does not update (the first colour: its share of all of them).
+// The iterate is read from L2 (ld.cg): up to three colours' kernels are in flight
+// and the first of them may have left lines of xd's buffer in an SM's L1.
+//
+// The inverse and the packed rows are copied to shared memory (cp.async) before
+// the wait for the previous colour's kernel (programmatic dependent launch), so
+// a colour is bound by the chain gather - residual - solve (and in FP64 by the
+// FP64 pipe: 18,700 FMA per 65-node patch, 8 us on one SM), not by its matrix
+// reads. A sliced residual launch and a local-solve launch per colour read A
+// three times and 32-bit columns. Loaded into registers instead of shared memory,
+// three patches fit an SM instead of four and the chains of the long rows stay
+// in the open: 17 us per colour.
+// One cycle on 24^3 cubes, mixed form (4 sweeps of 27 colours and the coarse
+// level): 2.2 ms with two launches per colour, 1.36 ms; on 12^3 cubes in FP64 3.13
+// and 1.80 ms. After the wait a block takes 3.6 us in FP32 (gather 1.1, residual
+// 1.0, solve 0.6), 11 us in FP64.
+//
+// out: the additive sweep; the corrections go to the local storage, x is only
+// read.
+struct NodalPack {
+  const int *vptr, *vidx, *voff, *ioff, *ch0, *hptr, *hnv, *halo;
+  const int64_t* aoff;
+  const uint2* chunk;
+  const unsigned char* row;
+  const unsigned short* idx;
+  const unsigned* mask;
+};
+
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+  const unsigned d = unsigned(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+constexpr int kNodalParts64 = 5;  // column parts of a row in the FP64 local solve
+
+// three values of a 16- or 32-byte group in shared memory
+__device__ __forceinline__ void load3(const float* p, float& a, float& b, float& c) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  a = v.x;
+  b = v.y;
+  c = v.z;
+}
+__device__ __forceinline__ void load3(const double* p, double& a, double& b, double& c) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  a = v.x;
+  b = v.y;
+  c = p[2];
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <class T, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, int prev_cnt,
+              const int* __restrict__ prev, int colour, int nu, int n, NodalPack pk, const T* __restrict__ vals,
+              const T* __restrict__ ainv, const T* __restrict__ tb, const T* __restrict__ sinv,
+              const T* __restrict__ cd, const T* __restrict__ b, const T* __restrict__ xs, T* __restrict__ xd,
+              T* __restrict__ out, T damp) {
+  constexpr int R = NT / 4, NW = NT / 32, PER = 16 / int(sizeof(T));
+  extern __shared__ __align__(16) unsigned char np_smem[];
+  __shared__ __align__(16) T rp[kNodalParts][R][4];  // partial row sums; [0] becomes the residual
+  __shared__ T part[(sizeof(T) == 8 ? kNodalParts64 : 4) * 3 * kNodalMaxNodes];
+  __shared__ T dot[NT];
+  pdl_trigger();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int i = patches ? patches[blockIdx.x] : int(blockIdx.x);
+  const int v0 = pk.vptr[i], m = pk.vptr[i + 1] - v0, rows3 = 3 * m;
+  const int vo = pk.voff[i], io = pk.ioff[i];
+  const int nv = pk.voff[i + 1] - vo, ni = pk.ioff[i + 1] - io;
+  const int c0 = pk.ch0[i], nch = pk.ch0[i + 1] - c0;
+  const int h0 = pk.hptr[i], nh = pk.hnv[i], nhp = pk.hptr[i + 1] - h0 - nh;
+  const T si = sinv[i], cdi = cd[i];
+  const int* nodes = pk.vidx + v0;
+  // shared memory: the packed values, the packed indices, the inverse
+  // (column-major), the halo's velocities [3][nh] and pressures
+  const int inv_n = (m * m + 3) & ~3;
+  T* sv = reinterpret_cast<T*>(np_smem);
+  unsigned short* sidx = reinterpret_cast<unsigned short*>(sv + 32 * nv);
+  T* sinvm = reinterpret_cast<T*>(sidx + 32 * ni);
+  T* hx = sinvm + inv_n;
+  T *hx1 = hx + nh, *hx2 = hx1 + nh, *hp = hx2 + nh;
+  {
+    const T* pv = vals + size_t(32) * vo;
+    for (int e = t; e < nv * 32 / PER; e += NT) copy_async16(sv + e * PER, pv + e * PER);
+    const unsigned short* pi = pk.idx + size_t(32) * io;
+    for (int e = t; e < ni * 4; e += NT) copy_async16(sidx + e * 8, pi + e * 8);
+    const T* A = ainv + pk.aoff[i];
+    for (int e = t; e < inv_n / PER; e += NT) copy_async16(sinvm + e * PER, A + e * PER);
+  }
+  for (int e = t; e < kNodalParts * R * 4; e += NT) (&rp[0][0][0])[e] = T(0);
+  // all A steps come before the B^T steps: nv = A + 3 B^T, ni = A + B^T
+  const int nb_steps = (nv - ni) / 2, na_steps = ni - nb_steps;
+  // everything else that the chain after the wait would have to fetch: the
+  // warp's first two chunks, the thread's velocity unknown (component t / m, node
+  // t % m) and its first two halo entries
+  constexpr int CP = 2;
+  uint2 chunk[CP];
+  int crow[CP];
+#pragma unroll
+  for (int u = 0; u < CP; ++u) {
+    const int ch = warp + u * NW;
+    chunk[u] = ch < nch ? pk.chunk[c0 + ch] : make_uint2(0, 0);
+    crow[u] = ch < nch ? pk.row[(c0 + ch) * 8 + (lane & 7)] : 255;
+  }
+  const int comp = t < rows3 ? t / m : 0, node = t < rows3 ? t - comp * m : 0;
+  T tt = T(0), bb = T(0);
+  int g = 0;
+  if (t < rows3) {
+    tt = tb[6 * size_t(v0) + t];
+    bb = tb[6 * size_t(v0) + rows3 + t];
+    g = comp * nu + nodes[node];
+  }
+  int gn[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) gn[u] = t + u * NT < nh + nhp ? pk.halo[h0 + t + u * NT] : 0;
+  // the thread's node of the previous colour's patch, if this colour leaves it
+  int pn = -1, pp = -1;
+  if (int(blockIdx.x) < prev_cnt) {
+    const int ip = prev[blockIdx.x], w0 = pk.vptr[ip], mp = pk.vptr[ip + 1] - w0;
+    if (t < mp) {
+      pn = pk.vidx[w0 + t];
+      if ((pk.mask[pn] >> colour) & 1u) pn = -1;
+    }
+    if (t == 0) pp = ip;
+  }
+  pdl_wait();
+  if (guarded(guard)) {  // uniform for the whole grid
+    // the first colour leaves x in both buffers, the later ones find it there
+    if (xd && prev_cnt < 0)
+      for (int e = blockIdx.x * NT + t; e < n; e += gridDim.x * NT) xd[e] = __ldcg(xs + e);
+    copy_async_wait();
+    return;
+  }
+  const T rhs = t < rows3 ? __ldcg(b + g) : T(0);
+  const T rhs_p = t == 0 ? __ldcg(b + 3 * nu + i) : T(0);
+  const T xp = t == 0 ? __ldcg(xs + 3 * nu + i) : T(0);
+  T c1 = T(0), c2 = T(0), c3 = T(0), c4 = T(0);
+  if (pn >= 0) {
+    c1 = __ldcg(xs + pn);
+    c2 = __ldcg(xs + nu + pn);
+    c3 = __ldcg(xs + 2 * nu + pn);
+  }
+  if (pp >= 0) c4 = __ldcg(xs + 3 * nu + pp);
+  // both halo entries' loads in flight before the first store
+  T hv[2][3];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int e = t + u * NT, k = e < nh ? gn[u] : 3 * nu + gn[u];
+    hv[u][0] = hv[u][1] = hv[u][2] = T(0);
+    if (e < nh + nhp) hv[u][0] = __ldcg(xs + k);
+    if (e < nh) {
+      hv[u][1] = __ldcg(xs + nu + k);
+      hv[u][2] = __ldcg(xs + 2 * nu + k);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int e = t + u * NT;
+    if (e < nh) {
+      hx[e] = hv[u][0];
+      hx1[e] = hv[u][1];
+      hx2[e] = hv[u][2];
+    } else if (e < nh + nhp) {
+      hp[e - nh] = hv[u][0];
+    }
+  }
+  for (int e = t + 2 * NT; e < nh + nhp; e += NT) {
+    const int k = pk.halo[h0 + e];
+    if (e < nh) {
+      hx[e] = __ldcg(xs + k);
+      hx1[e] = __ldcg(xs + nu + k);
+      hx2[e] = __ldcg(xs + 2 * nu + k);
+    } else {
+      hp[e - nh] = __ldcg(xs + 3 * nu + k);
+    }
+  }
+  if (pn >= 0) {
+    xd[pn] = c1;
+    xd[nu + pn] = c2;
+    xd[2 * nu + pn] = c3;
+  }
+  if (pp >= 0) xd[3 * nu + pp] = c4;
+  copy_async_wait();
+  __syncthreads();
+  auto residual_rows = [&](uint2 raw, int row) {
+    const int a0 = raw.x & 0xffff, b0 = raw.x >> 16, na = raw.y & 0xff, nb = (raw.y >> 8) & 0xff,
+              pt = (raw.y >> 16) & 0xff;
+    const int sub = lane >> 3;
+    T r0 = T(0), r1 = T(0), r2 = T(0);
+    const T* v = sv + 32 * a0 + lane;
+    const unsigned short* x = sidx + 32 * a0 + lane;
+    // every index before the first gather: the chain is two loads long
+    int k[kNodalSteps];
+#pragma unroll
+    for (int u = 0; u < kNodalSteps; ++u) k[u] = u < na ? int(x[32 * u]) : 0;
+#pragma unroll
+    for (int u = 0; u < kNodalSteps; ++u)
+      if (u < na) {
+        const T val = v[32 * u];
+        r0 += val * hx[k[u]];
+        r1 += val * hx1[k[u]];
+        r2 += val * hx2[k[u]];
+      }
+    v = sv + 32 * (na_steps + 3 * b0) + lane;
+    x = sidx + 32 * (na_steps + b0) + lane;
+    for (int u = 0; u < nb; ++u) {
+      const T pr = hp[x[32 * u]];
+      r0 += v[96 * u] * pr;
+      r1 += v[96 * u + 32] * pr;
+      r2 += v[96 * u + 64] * pr;
+    }
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1) {
+      r0 += __shfl_xor_sync(0xffffffffu, r0, o);
+      r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+      r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+    }
+    if (row != 255 && sub < 3) rp[pt][row][sub] = sub == 0 ? r0 : sub == 1 ? r1 : r2;
+  };
+#pragma unroll
+  for (int u = 0; u < CP; ++u)
+    if (warp + u * NW < nch) residual_rows(chunk[u], crow[u]);
+  for (int ch = warp + CP * NW; ch < nch; ch += NW)
+    residual_rows(pk.chunk[c0 + ch], pk.row[(c0 + ch) * 8 + (lane & 7)]);
+  __syncthreads();
+  if (t < rows3) {
+    T s = rhs - rp[0][node][comp];
+#pragma unroll
+    for (int k = 1; k < kNodalParts; ++k) s -= rp[k][node][comp];
+    rp[0][node][comp] = s;
+  }
+  __syncthreads();
+  // w = A^{-1} r: thread (q, a) sums the q-th part of row a's columns. FP64: as
+  // many parts as the block has threads for, rows packed (an FP64 instruction
+  // costs a warp the same for one active lane as for 32); FP32: four parts at
+  // fixed threads (no division, one part per warp and so one broadcast)
+  constexpr bool PACK = sizeof(T) == 8;
+  const int parts = PACK ? min(kNodalParts64, NT / m) : 4;
+  const int stride = PACK ? m : NT / 4;
+  if (t < parts * stride && t % stride < m) {
+    const int q = t / stride, a = t - q * stride;
+    const int qlen = (m + parts - 1) / parts, b0 = q * qlen, b1 = min(m, b0 + qlen);
+    T w0 = T(0), w1 = T(0), w2 = T(0);
+#pragma unroll 6
+    for (int k = b0; k < b1; ++k) {
+      const T av = sinvm[k * m + a];
+      T x0, x1, x2;
+      load3(&rp[0][k][0], x0, x1, x2);
+      w0 += av * x0;
+      w1 += av * x1;
+      w2 += av * x2;
+    }
+    T* to = part + q * rows3 + a;
+    to[0] = w0;
+    to[m] = w1;
+    to[2 * m] = w2;
+  }
+  __syncthreads();
+  T w = T(0), xo = T(0), d = T(0);
+  if (t < rows3) {
+    w = part[t];
+    for (int q = 1; q < parts; ++q) w += part[q * rows3 + t];
+    xo = hx[comp * nh + node];
+    d = bb * (xo + w);
+  }
+  // one warp sums the dot product: an FP64 addition costs a warp 75 clocks of
+  // its quarter's pipe, so ten warps with their own trees cost more
+  dot[t] = d;
+  __syncthreads();
+  if (warp == 0) {
+    T e[NW];
+#pragma unroll
+    for (int k = 0; k < NW; ++k) e[k] = dot[lane + 32 * k];
+#pragma unroll
+    for (int k = 1; k < NW; ++k)
+      if (32 * k < rows3) e[0] += e[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e[0] += __shfl_xor_sync(0xffffffffu, e[0], o);
+    // the pressure's own residual joins it
+    if (lane == 0) dot[0] = -si * (e[0] + (cdi * xp - rhs_p));
+  }
+  __syncthreads();
+  const T pr = dot[0];
+  const T du = damp * (w - tt * pr);
+  if (out) {
+    const size_t off = 3 * size_t(v0) + i;
+    if (t < rows3) out[off + t] = du;
+    if (t == 0) out[off + rows3] = damp * pr;
+    return;
+  }
+  if (t < rows3) xd[g] = xo + du;
+  if (t == 0) xd[3 * nu + i] = xp + damp * pr;
+  if (prev_cnt < 0) {
+    for (int e = blockIdx.x * NT + t; e < n; e += gridDim.x * NT) {
+      const int k = e < 3 * nu ? e % nu : e - 2 * nu;
+      if (!((pk.mask[k] >> colour) & 1u)) xd[e] = __ldcg(xs + e);
+    }
+    return;
+  }
+  // a previous colour with more patches than this one has
+  for (int j = blockIdx.x + gridDim.x; j < prev_cnt; j += gridDim.x) {
+    const int ip = prev[j], w0 = pk.vptr[ip], mp = pk.vptr[ip + 1] - w0;
+    for (int e = t; e < mp; e += NT) {
+      const int k = pk.vidx[w0 + e];
+      if ((pk.mask[k] >> colour) & 1u) continue;
+      xd[k] = __ldcg(xs + k);
+      xd[nu + k] = __ldcg(xs + nu + k);
+      xd[2 * nu + k] = __ldcg(xs + 2 * nu + k);
+    }
+    if (t == 0) xd[3 * nu + ip] = __ldcg(xs + 3 * nu + ip);
+  }
+}
+
+template <class T, int NT, int MINB>
+static void launch_nodal_patch_nt(pm_ctx* c, const DevNodalVanka& nv, int cnt, const int* patches, int prev_cnt,
+                                  const int* prev, int colour, const T* vals, const T* ainv, const T* tb,
+                                  const T* sinv, const T* cd, const T* b, const T* xs, T* xd, T* out, T damp) {
+  const NodalPack pk{nv.vptr.p,  nv.vidx.p,        nv.pk_voff.p, nv.pk_ioff.p,  nv.pk_ch0.p, nv.pk_hptr.p,
+                     nv.pk_hnv.p, nv.pk_halo_idx.p, nv.aoff.p,   nv.pk_chunk.p, nv.pk_row.p, nv.pk_idx.p,
+                     nv.pk_mask.p};
+  const std::vector<int>& need = sizeof(T) == 4 ? nv.pk_smem32 : nv.pk_smem64;
+  const size_t smem = size_t(patches ? need[size_t(colour)] : need.back());
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(k_nodal_patch<T, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    int(kNodalPatchSmem));
+  });
+  PM_CUDA(attr_err);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(cnt));
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c->pdl >= 1 ? 1 : 0;
+  PM_CUDA(cudaLaunchKernelEx(&cfg, k_nodal_patch<T, NT, MINB>, c->guard, patches, prev_cnt, prev, colour, nv.nu, nv.n,
+                             pk, vals, ainv, tb, sinv, cd, b, xs, xd, out, damp));
+  c->kernel_launches++;
+}
+
+// 12 warps: one chunk of the residual each for most patches
+template <class T, class... Args>
+static void launch_nodal_patch(pm_ctx* c, const DevNodalVanka& nv, Args... args) {
+  static_assert(4 * kNodalMaxNodes <= 384, "four threads per row, one per velocity unknown");
+  launch_nodal_patch_nt<T, 384, sizeof(T) == 4 ? 3 : 1>(c, nv, args...);
+}
+
 template <class T>
-static void nodal_jacobi(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T* ainv, const T* tb, const T* sinv,
-                         T* sol, const T* b, T* x, T* r, T damp) {
-  if constexpr (sizeof(T) == 8) csr_apply(c, V, EPI_DEFECT, x, r, b, 1.0);
-  else csr_apply32(c, V, EPI_DEFECT, x, r, b, 1.0f);
-  k_nodal_local<T><<<nv.np, kLocalThreads, 0, c->stream>>>(c->guard, nv.np, nullptr, nv.nu, nv.vptr.p, nv.vidx.p, nv.aoff.p,
-                                                          ainv, tb, sinv, r, nullptr, sol, nullptr, damp);
+static void nodal_jacobi(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T* vals, const T* ainv, const T* tb,
+                         const T* sinv, const T* cd, T* sol, const T* b, T* x, T* r, T damp) {
+  if (nv.pk_ok && vals && c->nodal_sliced == 8) {
+    launch_nodal_patch<T>(c, nv, nv.np, nullptr, 0, nullptr, 0, vals, ainv, tb, sinv, cd, b, (const T*)x, nullptr,
+                          sol, damp);
+  } else {
+    if constexpr (sizeof(T) == 8) csr_apply(c, V, EPI_DEFECT, x, r, b, 1.0);
+    else csr_apply32(c, V, EPI_DEFECT, x, r, b, 1.0f);
+    k_nodal_local<T><<<nv.np, kLocalThreads, 0, c->stream>>>(c->guard, nv.np, nullptr, nv.nu, nv.vptr.p, nv.vidx.p,
+                                                            nv.aoff.p, ainv, tb, sinv, r, nullptr, sol, nullptr,
+                                                            damp);
+    c->kernel_launches++;
+  }
   const int g = std::max(1, std::min((nv.n + 255) / 256, c->num_sms * 16));
   k_vanka_average<T><<<g, 256, 0, c->stream>>>(c->guard, nv.n, nv.inc_ptr.p, nv.inc_idx.p, nv.count.p, sol, x);
   PM_CHECK_LAUNCH();
-  c->kernel_launches += 2;
+  c->kernel_launches++;
 }
 
 // bloc[slot] = b[global row of the slot]
@@ -1654,8 +2207,9 @@ __global__ void k_gather_slots(const int* __restrict__ guard, int n, const int* 
 }
 
 template <class T>
-static void nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T* vals, const T* ainv, const T* tb,
-                          const T* sinv, T* rloc, const T* b, T* x, T damp) {
+static bool nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T* vals, const T* packed,
+                          const T* ainv, const T* tb, const T* sinv, const T* cd, T* rloc, const T* b, T* x,
+                          T* other, T damp) {
   const int ncol = int(nv.color_ptr.size()) - 1;
   const T* rsv = nullptr;
   T* bl = nullptr;
@@ -1666,16 +2220,20 @@ static void nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T
     rsv = nv.rs_vals.p;
     bl = nv.bloc.p;
   }
+  const bool fused = nv.pk_ok && packed && other && c->nodal_sliced == 8;
   const bool sliced = nv.rs_ok && rsv && bl && c->nodal_sliced != 0;
   BlockMask mg{};
   mg.guard = c->guard;
-  if (sliced) {
+  if (!fused && sliced) {
     const int n = int(nv.bslot.n);
     const int g = std::max(1, std::min((n + 255) / 256, c->num_sms * 8));
     k_gather_slots<T><<<g, 256, 0, c->stream>>>(c->guard, n, nv.bslot.p, b, bl);
     PM_CHECK_LAUNCH();
     c->kernel_launches++;
   }
+  bool moved = false;      // the iterate is in `other`
+  int prev_cnt = -1;       // the first colour writes every entry of its target
+  const int* prev = nullptr;
   for (int k = 0; k < ncol; ++k) {
     const int beg = nv.color_ptr[k], cnt = nv.color_ptr[k + 1] - beg;
     if (!cnt) continue;
@@ -1690,6 +2248,19 @@ static void nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T
       const double eb = double(sizeof(T));
       c->probe_bytes.push_back(double(nv.color_entries[k]) * (2 * eb + 4) + double(nv.color_rows[k]) * 5 * eb +
                                double(nv.color_msq[k]) * eb + double(nv.color_nodes[k]) * 6 * eb + double(cnt) * eb);
+    }
+    if (fused) {
+      launch_nodal_patch<T>(c, nv, cnt, pts, prev_cnt, prev, k, packed, ainv, tb, sinv, cd, b,
+                            (const T*)(moved ? other : x), moved ? x : other, nullptr, damp);
+      moved = !moved;
+      prev_cnt = cnt;
+      prev = pts;
+      if (c->probe_nodal) {
+        cudaEvent_t e1 = probe_event(c);
+        PM_CUDA(cudaEventRecord(e1, c->stream));
+        c->probe_events.push_back(e1);
+      }
+      continue;
     }
     if (sliced) {
       // the colour's local residuals as one sliced SpMV: rloc[slot] = bloc[slot] - (V x)[row]
@@ -1714,19 +2285,22 @@ static void nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T
     }
   }
   PM_CHECK_LAUNCH();
+  return moved;
 }
 
 void DevNodalVanka::sweep_jacobi(pm_ctx* c, const DevCsr& V, const double* b, double* x, double* r, double damp) {
-  nodal_jacobi<double>(c, *this, V, ainv.p, tb.p, sinv.p, sol.p, b, x, r, damp);
+  nodal_jacobi<double>(c, *this, V, pk_vals.p, ainv.p, tb.p, sinv.p, cdiag.p, sol.p, b, x, r, damp);
 }
 void DevNodalVanka::sweep_jacobi32(pm_ctx* c, const DevCsr& V, const float* b, float* x, float* r, float damp) {
-  nodal_jacobi<float>(c, *this, V, ainv32.p, tb32.p, sinv32.p, sol32.p, b, x, r, damp);
+  nodal_jacobi<float>(c, *this, V, pk_vals32.p, ainv32.p, tb32.p, sinv32.p, cdiag32.p, sol32.p, b, x, r, damp);
 }
-void DevNodalVanka::sweep_colored(pm_ctx* c, const DevCsr& V, const double* b, double* x, double damp) {
-  nodal_colored<double>(c, *this, V, V.vals.p, ainv.p, tb.p, sinv.p, sol.p, b, x, damp);
+bool DevNodalVanka::sweep_colored(pm_ctx* c, const DevCsr& V, const double* b, double* x, double* other, double damp) {
+  return nodal_colored<double>(c, *this, V, V.vals.p, pk_vals.p, ainv.p, tb.p, sinv.p, cdiag.p, sol.p, b, x, other,
+                               damp);
 }
-void DevNodalVanka::sweep_colored32(pm_ctx* c, const DevCsr& V, const float* b, float* x, float damp) {
-  nodal_colored<float>(c, *this, V, V.vals32.p, ainv32.p, tb32.p, sinv32.p, sol32.p, b, x, damp);
+bool DevNodalVanka::sweep_colored32(pm_ctx* c, const DevCsr& V, const float* b, float* x, float* other, float damp) {
+  return nodal_colored<float>(c, *this, V, V.vals32.p, pk_vals32.p, ainv32.p, tb32.p, sinv32.p, cdiag32.p, sol32.p, b,
+                              x, other, damp);
 }
 
 }  // namespace pm

@@ -176,6 +176,23 @@ struct DevNodalVanka {
   DBuf<int> rs_perm, rs_off, rs_cols, rs_src, bslot;
   DBuf<float> rs_vals32, bloc32;
   DBuf<double> rs_vals, bloc;
+  // the patches packed for k_nodal_patch (see there), when they fit it
+  bool pk_ok = false;
+  // per colour and (last entry) over all patches: shared memory of a block, for
+  // FP32 and FP64 values
+  std::vector<int> pk_smem32, pk_smem64;
+  int64_t pk_entries = 0;               // packed values
+  DBuf<int> pk_voff, pk_ioff;           // per patch: values and indices, in units of 32 (np + 1)
+  DBuf<uint2> pk_chunk;                 // NodalChunk of every warp's share
+  DBuf<int> pk_ch0, pk_hptr, pk_hnv;    // per patch: first chunk, halo list, its velocity nodes
+  DBuf<unsigned char> pk_row;           // patch row at each chunk position, 255 = none
+  DBuf<unsigned short> pk_idx;          // halo index of each entry
+  DBuf<int> pk_halo_idx, pk_src;        // halo nodes (velocity, then pressure); CSR entry of each value
+  DBuf<unsigned> pk_mask;               // colours of the patches holding a velocity node / of a pressure
+  DBuf<double> pk_vals, cdiag;          // packed values; the pressures' own diagonal entries
+  DBuf<float> pk_vals32, cdiag32;
+  bool build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vector<int>& vp, const std::vector<int>& vi,
+                  const std::vector<int>& color, int n_colors);
   void setup(pm_ctx* c, const DiscLevel& L);
   void build_row_slices(pm_ctx* c, const pmsetup::Csr& S, int p0, const std::vector<int>& vp,
                         const std::vector<int>& vi, const std::vector<int>& cp);
@@ -183,9 +200,10 @@ struct DevNodalVanka {
   // additive sweep: x += average of damp * local corrections from one residual
   void sweep_jacobi(pm_ctx* c, const DevCsr& V, const double* b, double* x, double* r, double damp);
   void sweep_jacobi32(pm_ctx* c, const DevCsr& V, const float* b, float* x, float* r, float damp);
-  // multiplicative sweep, patches grouped by colour
-  void sweep_colored(pm_ctx* c, const DevCsr& V, const double* b, double* x, double damp);
-  void sweep_colored32(pm_ctx* c, const DevCsr& V, const float* b, float* x, float damp);
+  // multiplicative sweep, patches grouped by colour; other: a second vector of
+  // x's size. True: the new iterate is in `other`, false: in x
+  bool sweep_colored(pm_ctx* c, const DevCsr& V, const double* b, double* x, double* other, double damp);
+  bool sweep_colored32(pm_ctx* c, const DevCsr& V, const float* b, float* x, float* other, float damp);
 };
 
 }  // namespace pm
