@@ -724,30 +724,8 @@ static void launch_elem_qk(pm_ctx* c, int n_cells, const double* verts, const De
 }
 
 // Stage 2: CSR values and right-hand side from the element matrices and
-// vectors, each entry summing its contributions in cell order. An entry
-// without contributions is a Dirichlet row's diagonal (1) or right-hand side
-// (0). Four index loads and then four value loads of an entry are in flight
-// at a time; one launch for the matrix and the right-hand side (three with a
-// pass for the unit diagonals). Bound by the scattered reads of the element
-// matrices.
-__device__ __forceinline__ double gather_entry(const int* __restrict__ idx, const double* __restrict__ K, int beg,
-                                               int end) {
-  constexpr int U = 4;
-  double s = 0.0;
-  for (int t = beg; t < end; t += U) {
-    int k[U];
-    double v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) k[u] = t + u < end ? __ldg(idx + t + u) : -1;
-#pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = k[u] >= 0 ? __ldg(K + k[u]) : 0.0;
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (t + u < end) s += v[u];
-  }
-  return s;
-}
-
+// vectors (gather_entry); one launch for the matrix and the right-hand side
+// (three with a pass for the unit diagonals).
 __global__ void __launch_bounds__(256) k_gather(int nnz, const int* __restrict__ ptr, const int* __restrict__ idx,
                                                 const double* __restrict__ K, double* __restrict__ vals, int n,
                                                 const int* __restrict__ rptr, const int* __restrict__ ridx,

@@ -7,6 +7,29 @@
 
 namespace pm {
 
+// Stage 2 of an assembly: an entry of the matrix or the right-hand side sums its
+// contributions in cell order. An entry without contributions is a Dirichlet
+// row's diagonal (1) or right-hand side (0). Four index loads and then four value
+// loads of an entry are in flight at a time. Bound by the scattered reads of the
+// element matrices.
+__device__ __forceinline__ double gather_entry(const int* __restrict__ idx, const double* __restrict__ K, int beg,
+                                               int end) {
+  constexpr int U = 4;
+  double s = 0.0;
+  for (int t = beg; t < end; t += U) {
+    int k[U];
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) k[u] = t + u < end ? __ldg(idx + t + u) : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = k[u] >= 0 ? __ldg(K + k[u]) : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t + u < end) s += v[u];
+  }
+  return s;
+}
+
 // reference-element tables of a Qk element on a tensor Gauss rule
 // 1D tables of a tensor-product element (Q1, Q2) on its Gauss rule, K1 = k + 1
 // basis functions: M_ij = sum_q w phi_i phi_j, S_ij = sum_q w phi_i' phi_j',

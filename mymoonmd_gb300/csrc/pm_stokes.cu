@@ -19,6 +19,7 @@
 #include <numeric>
 #include <vector>
 
+#include "pm_assemble.h"
 #include "pm_stokes.h"
 #include "pm_tetra.h"
 
@@ -27,12 +28,12 @@ namespace pm {
 // ------------------------------------------------------------- tables ------
 // the P4Tetra / P5Tetra rules and the P2 basis: pm_tetra.h
 
-// layout: S[6][100] | D[3][40] | phi2[qn][10] | w[qn] | xi[qn][3] | C[3][10][10][10]
+// layout: S[6][100] | D[3][40] | phi2[qn][10] | w[qn] | xi[qn][3] | C[10][4][10]
 static constexpr int kOffS = 0, kOffD = 600, kOffPhi = 720;
 __host__ __device__ constexpr int tab_off_w(int qn) { return kOffPhi + 10 * qn; }
 __host__ __device__ constexpr int tab_off_xi(int qn) { return tab_off_w(qn) + qn; }
 __host__ __device__ constexpr int tab_off_c(int qn) { return tab_off_xi(qn) + 3 * qn; }
-__host__ __device__ constexpr int tab_size(int qn) { return tab_off_c(qn) + 3000; }
+__host__ __device__ constexpr int tab_size(int qn) { return tab_off_c(qn) + 400; }
 
 void DevStokesTables::upload(pm_ctx* c, int nq, bool skew) {
   if (nq != kP4n && nq != kP5n) throw Error(PM_E_UNSUPPORTED, "Stokes tables: 11 or 15 quadrature points");
@@ -77,21 +78,17 @@ void DevStokesTables::upload(pm_ctx* c, int nq, bool skew) {
     t[tab_off_xi(nq) + q * 3 + 1] = qy[q];
     t[tab_off_xi(nq) + q * 3 + 2] = qz[q];
   }
-  // C[a][i][j][k]: test function i, ansatz function j (derivative a), velocity
-  // basis function k; for the skew-symmetric form (1/2) [((u.grad) phi_j,
-  // phi_i) - ((u.grad) phi_i, phi_j)] (NSNonlinearTerm_skew_symmetric) its
-  // antisymmetric part in (i, j)
-  auto conv = [&](int a, int i, int j, int l) {
-    double s = 0.0;
-    for (int q = 0; q < nq; ++q) s += qw[q] * phi[q * 10 + i] * D(a, q, j) * phi[q * 10 + l];
-    return s;
-  };
-  for (int a = 0; a < 3; ++a)
-    for (int i = 0; i < 10; ++i)
-      for (int j = 0; j < 10; ++j)
-        for (int l = 0; l < 10; ++l)
-          t[tab_off_c(nq) + a * 1000 + i * 100 + j * 10 + l] =
-              skew ? 0.5 * (conv(a, i, j, l) - conv(a, j, i, l)) : conv(a, i, j, l);
+  // C[i][l][k] = sum_q w phi_i lambda_l phi_k: test function i, barycentric
+  // coordinate l (the gradient of an ansatz function is linear), velocity basis
+  // function k
+  for (int i = 0; i < 10; ++i)
+    for (int l = 0; l < 4; ++l)
+      for (int k2 = 0; k2 < 10; ++k2) {
+        double s = 0.0;
+        for (int q = 0; q < nq; ++q) s += qw[q] * phi[q * 10 + i] * psi[q * 4 + l] * phi[q * 10 + k2];
+        t[tab_off_c(nq) + (i * 4 + l) * 10 + k2] = s;
+      }
+  skew_form = skew;
   data.upload(t, c->stream);
 }
 
@@ -103,7 +100,6 @@ void DevStokesLevel::upload(pm_ctx* c, const DiscLevel& L) {
   gat_idx.upload(L.gat_idx, c->stream);
   rgat_ptr.upload(L.rgat_ptr, c->stream);
   rgat_idx.upload(L.rgat_idx, c->stream);
-  diag_pos.upload(L.diag_pos, c->stream);
   nvel = L.block_len[0];
   nvel_active = L.block_active[0];
   np = L.block_len[3];
@@ -165,10 +161,10 @@ __device__ void stokes_f(double nu, const double* x, double* f, int example, boo
   const double p = 3.14159265358979323846;
   double S[3], S1[3], S2[3], S3[3];
   for (int d = 0; d < 3; ++d) {
+    // sin and cos of 2 pi t by the double angle: one sincospi per coordinate
     double s, c;
     sincospi(x[d], &s, &c);
-    double s2, c2;
-    sincospi(2.0 * x[d], &s2, &c2);
+    const double s2 = 2.0 * s * c, c2 = 1.0 - 2.0 * s * s;
     S[d] = s * s;                    // sin^2(pi t)
     S1[d] = p * s2;                  // d/dt
     S2[d] = 2 * p * p * c2;          // d2/dt2
@@ -184,17 +180,29 @@ __device__ void stokes_f(double nu, const double* x, double* f, int example, boo
   f[2] = -nu * (lx - ly) + 1.0;
 }
 
+// entry (i, j) of the convective term from U (see k_elem_stokes); local DOF order
+// v0, m01, v1, m02, m12, v2, m03, m13, m23, v3
+__device__ __forceinline__ double p2_convection(const double (*U)[10][4], int i, int j) {
+  // the vertices (p, q) of the function's edge, p = q for a vertex
+  const int pq = j == 0 ? 0x00 : j == 1 ? 0x01 : j == 2 ? 0x11 : j == 3 ? 0x02 : j == 4 ? 0x12 : j == 5 ? 0x22
+               : j == 6 ? 0x03 : j == 7 ? 0x13 : j == 8 ? 0x23 : 0x33;
+  const int p = pq >> 4, q = pq & 15;
+  if (p == q) return 4.0 * U[p][i][p] - ((U[p][i][0] + U[p][i][1]) + (U[p][i][2] + U[p][i][3]));
+  return 4.0 * (U[q][i][p] + U[p][i][q]);
+}
+
 // one block per CHUNK cells: per-cell geometry factors, then the element
 // matrix as contractions of the reference tensors (A part: stiffness and,
 // with a velocity u, the convective term; B part) and, with F, the element
 // right-hand side on the NQ-point rule
-template <int CHUNK, int NQ>
+template <int CHUNK, int NQ, bool CONV>
 __global__ void __launch_bounds__(256) k_elem_stokes(int n_cells, const double* __restrict__ verts,
                                                      const double* __restrict__ tab, double nu,
                                                      double* __restrict__ K, double* __restrict__ F, int example,
                                                      bool convective_f, const double* __restrict__ u,
-                                                     const int* __restrict__ udof, int nvel) {
+                                                     const int* __restrict__ udof, int nvel, bool skew) {
   constexpr int kW = tab_off_w(NQ), kXi = tab_off_xi(NQ), kC = tab_off_c(NQ);
+  __shared__ double cU[CONV ? CHUNK : 1][4][10][4];  // see the convective term below
   __shared__ double cS[CHUNK][6];
   __shared__ double cB[CHUNK][9];
   __shared__ double geo[CHUNK][13];
@@ -246,7 +254,7 @@ __global__ void __launch_bounds__(256) k_elem_stokes(int n_cells, const double* 
     geo[t][12] = adet;
   }
   __syncthreads();
-  if (u) {
+  if (CONV) {
     for (int e = t; e < nc * 30; e += blockDim.x) {
       const int cl = e / 30, ak = e % 30, a = ak / 10, k = ak % 10;
       const int g = udof[(size_t)(c0 + cl) * 10 + k];
@@ -271,29 +279,61 @@ __global__ void __launch_bounds__(256) k_elem_stokes(int n_cells, const double* 
     }
   }
   __syncthreads();
-  for (int e = t; e < nc * 220; e += blockDim.x) {
-    const int cl = e / 220, p = e % 220;
-    double s = 0.0;
-    if (p < 100) {
+  // The convective term N_ij = sum_a sum_k V[a][k] int phi_i phi_k d_a phi_j.
+  // The gradient of a P2 function is linear, with barycentric coordinates
+  // lambda_b (d_a lambda_b = delta, lambda_0: -1): with
+  //   U_b[i][l] = sum_k V_b[k] C[i][l][k],  U_0 = -(U_1 + U_2 + U_3),
+  // a vertex function j = v gives 4 U_v[i][v] - sum_l U_v[i][l] and the edge
+  // function of (p, q) 4 (U_q[i][p] + U_p[i][q]): 1,560 operations per cell
+  // instead of the 3,000 of the sum over a and k for every (i, j).
+  if (CONV) {
+    if (t < 240) {
+      const int il = t % 40;
+      double tc[10];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) s = fma(cS[cl][k], __ldg(tab + kOffS + k * 100 + p), s);
-      if (u) {
-        // N_ij = sum_a sum_k V[a][k] C[a][i][j][k], p = i * 10 + j
-        double nsum = 0.0;
+      for (int k = 0; k < 10; ++k) tc[k] = __ldg(tab + kC + il * 10 + k);
+      for (int cl = t / 40; cl < nc; cl += 6) {
+        double s[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const double* Ca = tab + kC + a * 1000 + p * 10;
+        for (int a = 0; a < 3; ++a)
 #pragma unroll
-          for (int k = 0; k < 10; ++k) nsum = fma(cV[cl][a * 10 + k], __ldg(Ca + k), nsum);
-        }
-        s += nsum;
+          for (int k = 0; k < 10; ++k) s[a] = fma(cV[cl][a * 10 + k], tc[k], s[a]);
+        double* U = &cU[cl][0][0][0] + il;
+        U[0] = -(s[0] + s[1] + s[2]);
+        U[40] = s[0];
+        U[80] = s[1];
+        U[120] = s[2];
       }
-    } else {
-      const int kk = (p - 100) / 40, ij = (p - 100) % 40;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) s = fma(cB[cl][kk * 3 + a], __ldg(tab + kOffD + a * 40 + ij), s);
     }
-    K[(size_t)(c0 + cl) * 220 + p] = s;
+    __syncthreads();
+  }
+  // A: a thread keeps the 6 stiffness tensor values of one entry in registers
+  // and walks the cells. FP64 multiply-adds bound the kernel: 12^3 cubes with the
+  // convective term 130 us with 30 products per entry, 81 with these.
+  double* Kc = K + (size_t)c0 * 220;
+  if (t < 200) {
+    const int p = t % 100, tg = t / 100, i = p / 10, j = p % 10;
+    double ts[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) ts[k] = __ldg(tab + kOffS + k * 100 + p);
+    for (int cl = tg; cl < nc; cl += 2) {
+      double s = 0.0;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s = fma(cS[cl][k], ts[k], s);
+      if (CONV) {
+        double n = p2_convection(cU[cl], i, j);
+        if (skew) n = 0.5 * (n - p2_convection(cU[cl], j, i));  // the skew-symmetric form
+        s += n;
+      }
+      Kc[(size_t)cl * 220 + p] = s;
+    }
+  }
+  for (int e = t; e < nc * 120; e += blockDim.x) {
+    const int cl = e / 120, p = e % 120, kk = p / 40, ij = p % 40;
+    double s = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) s = fma(cB[cl][kk * 3 + a], __ldg(tab + kOffD + a * 40 + ij), s);
+    Kc[(size_t)cl * 220 + 100 + p] = s;
   }
   if (F) {
     for (int e = t; e < nc * 34; e += blockDim.x) {
@@ -308,18 +348,18 @@ __global__ void __launch_bounds__(256) k_elem_stokes(int n_cells, const double* 
   }
 }
 
-__global__ void k_gather_stokes(int nnz, const int* __restrict__ ptr, const int* __restrict__ idx,
-                                const double* __restrict__ K, double* __restrict__ vals) {
+// matrix values and (n > 0) the right-hand side from the element storage
+__global__ void __launch_bounds__(256) k_gather_stokes(int nnz, const int* __restrict__ ptr,
+                                                       const int* __restrict__ idx, const double* __restrict__ K,
+                                                       double* __restrict__ vals, int n,
+                                                       const int* __restrict__ rptr, const int* __restrict__ ridx,
+                                                       const double* __restrict__ F, double* __restrict__ rhs) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int t = ptr[e]; t < ptr[e + 1]; ++t) s += K[idx[t]];
-    vals[e] = s;
+    const int beg = __ldg(ptr + e), end = __ldg(ptr + e + 1);
+    vals[e] = beg < end ? gather_entry(idx, K, beg, end) : 1.0;
   }
-}
-
-__global__ void k_unit_diag(int n, const int* __restrict__ pos, double* __restrict__ vals) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) vals[pos[i]] = 1.0;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
+    rhs[e] = gather_entry(ridx, F, __ldg(rptr + e), __ldg(rptr + e + 1));
 }
 
 // Dirichlet values of example -3 at the non-active velocity DOFs of the three
@@ -334,18 +374,34 @@ __global__ void k_stokes_dirichlet(int nb, int nvel, int nact, const double* __r
   rhs[2 * nvel + nact + i] = -y * y;
 }
 
-static void launch_elem_stokes(pm_ctx* c, const DevStokesLevel& L, const DevStokesTables& t, double nu,
-                               double* K, double* F, int example, bool convective_f, const double* u) {
-  constexpr int CHUNK = 32;
+template <int NQ, int CHUNK>
+static void launch_elem_stokes_chunk(pm_ctx* c, const DevStokesLevel& L, const DevStokesTables& t, double nu, double* K,
+                                     double* F, int example, bool convective_f, const double* u) {
   const int g = (L.n_cells + CHUNK - 1) / CHUNK;
-  if (t.qn == kP4n)
-    k_elem_stokes<CHUNK, kP4n><<<g, 256, 0, c->stream>>>(L.n_cells, L.verts.p, t.data.p, nu, K, F, example,
-                                                          convective_f, u, L.udof.p, L.nvel);
+  if (u)
+    k_elem_stokes<CHUNK, NQ, true><<<g, 256, 0, c->stream>>>(L.n_cells, L.verts.p, t.data.p, nu, K, F, example,
+                                                              convective_f, u, L.udof.p, L.nvel, t.skew_form);
   else
-    k_elem_stokes<CHUNK, kP5n><<<g, 256, 0, c->stream>>>(L.n_cells, L.verts.p, t.data.p, nu, K, F, example,
-                                                          convective_f, u, L.udof.p, L.nvel);
+    k_elem_stokes<CHUNK, NQ, false><<<g, 256, 0, c->stream>>>(L.n_cells, L.verts.p, t.data.p, nu, K, F, example,
+                                                               convective_f, u, L.udof.p, L.nvel, t.skew_form);
   PM_CHECK_LAUNCH();
   c->kernel_launches++;
+}
+
+// cells per block: a block's FP64 work takes about 1.5 us per cell on its SM, so
+// levels of fewer than 16 cells per SM take blocks of 4 (1,296 cells: 24.5 us with
+// 16, 17.7 with 4; 10,368 cells within 3 % with 8 and 16)
+template <int NQ>
+static void launch_elem_stokes_rule(pm_ctx* c, const DevStokesLevel& L, const DevStokesTables& t, double nu, double* K,
+                                    double* F, int example, bool convective_f, const double* u) {
+  if (L.n_cells <= 16 * c->num_sms) launch_elem_stokes_chunk<NQ, 4>(c, L, t, nu, K, F, example, convective_f, u);
+  else launch_elem_stokes_chunk<NQ, 16>(c, L, t, nu, K, F, example, convective_f, u);
+}
+
+static void launch_elem_stokes(pm_ctx* c, const DevStokesLevel& L, const DevStokesTables& t, double nu,
+                               double* K, double* F, int example, bool convective_f, const double* u) {
+  if (t.qn == kP4n) launch_elem_stokes_rule<kP4n>(c, L, t, nu, K, F, example, convective_f, u);
+  else launch_elem_stokes_rule<kP5n>(c, L, t, nu, K, F, example, convective_f, u);
 }
 
 // element storage -> matrix values (and right-hand side)
@@ -353,19 +409,11 @@ static void gather_stokes(pm_ctx* c, const DevStokesLevel& L, DevCsr& A, double*
                           const double* F, int example) {
   const int nnz = int(A.nnz);
   const int g = std::max(1, std::min((nnz + 255) / 256, c->num_sms * 16));
-  k_gather_stokes<<<g, 256, 0, c->stream>>>(nnz, L.gat_ptr.p, L.gat_idx.p, K, A.vals.p);
+  k_gather_stokes<<<g, 256, 0, c->stream>>>(nnz, L.gat_ptr.p, L.gat_idx.p, K, A.vals.p, rhs ? L.n : 0, L.rgat_ptr.p,
+                                            L.rgat_idx.p, F, rhs);
   PM_CHECK_LAUNCH();
-  const int nd = int(L.diag_pos.n);
-  if (nd) {
-    k_unit_diag<<<(nd + 255) / 256, 256, 0, c->stream>>>(nd, L.diag_pos.p, A.vals.p);
-    PM_CHECK_LAUNCH();
-  }
-  c->kernel_launches += nd ? 2 : 1;
+  c->kernel_launches++;
   if (rhs) {
-    const int gr = std::max(1, std::min((L.n + 255) / 256, c->num_sms * 16));
-    k_gather_stokes<<<gr, 256, 0, c->stream>>>(L.n, L.rgat_ptr.p, L.rgat_idx.p, F, rhs);
-    PM_CHECK_LAUNCH();
-    c->kernel_launches++;
     const int nb = L.nvel - L.nvel_active;
     if (example == -3 && nb > 0) {
       k_stokes_dirichlet<<<(nb + 255) / 256, 256, 0, c->stream>>>(nb, L.nvel, L.nvel_active, L.bnd_xyz.p, rhs);
@@ -520,11 +568,13 @@ void restrict_velocity(pm_ctx* c, const DevStokesLevel& coarse, const DevStokesL
                        const double* u_fine, double* u_coarse, double* cellval) {
   if (!coarse.children.p) throw Error(PM_E_INVALID, "restriction: the coarse level has no children map");
   const int nw = coarse.n_cells * 30;
-  k_restrict_cells<<<(nw + 255) / 256, 256, 0, c->stream>>>(coarse.n_cells, coarse.children.p, fine.udof.p, q,
+  // blocks of 64 threads: a few thousand threads of long gather chains spread
+  // over all SMs
+  k_restrict_cells<<<(nw + 63) / 64, 64, 0, c->stream>>>(coarse.n_cells, coarse.children.p, fine.udof.p, q,
                                                             u_fine, fine.nvel, cellval);
   PM_CHECK_LAUNCH();
   const int nd = 3 * coarse.nvel;
-  k_restrict_average<<<(nd + 255) / 256, 256, 0, c->stream>>>(coarse.nvel, coarse.vinc_ptr.p, coarse.vinc_idx.p,
+  k_restrict_average<<<(nd + 63) / 64, 64, 0, c->stream>>>(coarse.nvel, coarse.vinc_ptr.p, coarse.vinc_idx.p,
                                                               cellval, u_coarse);
   PM_CHECK_LAUNCH();
   c->kernel_launches += 2;

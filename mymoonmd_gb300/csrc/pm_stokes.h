@@ -12,9 +12,9 @@ namespace pm {
 // otherwise)
 struct DevStokesTables {
   int qn = 11;
-  // S (6 x 100), D (3 x 40), phi2 (qn x 10), w (qn), xi (qn x 3), and the
-  // convection tensor C[a][i][j][k] = sum_q w phi_i d_a phi_j phi_k (3 x 1000;
-  // with skew its antisymmetric part in i, j: the skew-symmetric form)
+  // S (6 x 100), D (3 x 40), phi2 (qn x 10), w (qn), xi (qn x 3), and for the
+  // convective term C[i][l][k] = sum_q w phi_i lambda_l phi_k (10 x 4 x 10)
+  bool skew_form = false;  // the antisymmetric part of the convective term
   DBuf<double> data;
   void upload(pm_ctx* c, int qn = 11, bool skew = false);
 };
@@ -26,7 +26,7 @@ struct DevStokesLevel {
   int np = 0;                     // pressure DOFs
   DBuf<double> verts;
   DBuf<double> bnd_xyz;  // coordinates of the non-active velocity DOFs
-  DBuf<int> gat_ptr, gat_idx, rgat_ptr, rgat_idx, diag_pos;
+  DBuf<int> gat_ptr, gat_idx, rgat_ptr, rgat_idx;
   DBuf<int> udof;        // velocity GlobalNumbers (n_cells x 10)
   // P1 pressure: integral weights (sum over the cells of a DOF of |K| / 4)
   // and the measure of the domain, for the projection into L2_0
