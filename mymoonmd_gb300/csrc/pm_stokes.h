@@ -185,6 +185,7 @@ struct DevNodalVanka {
   DBuf<int> pk_voff, pk_ioff;           // per patch: values and indices, in units of 32 (np + 1)
   DBuf<uint2> pk_chunk;                 // NodalChunk of every warp's share
   DBuf<int> pk_ch0, pk_hptr, pk_hnv;    // per patch: first chunk, halo list, its velocity nodes
+  DBuf<int> pk_self;                    // per patch: its own pressure in the halo's pressures
   DBuf<unsigned char> pk_row;           // patch row at each chunk position, 255 = none
   DBuf<unsigned short> pk_idx;          // halo index of each entry
   DBuf<int> pk_halo_idx, pk_src;        // halo nodes (velocity, then pressure); CSR entry of each value
