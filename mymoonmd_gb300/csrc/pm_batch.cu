@@ -438,7 +438,7 @@ std::vector<BatchDone> BatchEngine::cycle(const std::vector<pm_problem*>& join) 
     nonactive_nonzero_batch(c, B, nw, A(L - 1).mask, r, at<int>(off_flags) + 2);
   }
   dot_partials_batch(c, B, cyc, n, r, r, at<double>(off_pA));
-  finish_sum_batch(c, B, cyc, at<double>(off_pA), at<double>(off_dres), true);
+  finish_sum_batch(c, B, cyc, n, at<double>(off_pA), at<double>(off_dres), true);
   PM_CUDA(cudaMemcpy2DAsync(hres, sizeof(double), block.p + off_dres, S, sizeof(double), size_t(B),
                             cudaMemcpyDeviceToHost, c->stream));
   PM_CUDA(cudaMemcpy2DAsync(hflag, sizeof(int) * 4, block.p + off_flags, S, sizeof(int) * 4, size_t(B),

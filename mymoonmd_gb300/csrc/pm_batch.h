@@ -69,11 +69,12 @@ void coarse_solve_batch(pm_ctx* c, int n_slots, const Batch& bt, const DenseInve
                         double* x);
 void coarse_solve32_batch(pm_ctx* c, int n_slots, const Batch& bt, const DenseInverse& inv0, const float* b,
                           float* x);
-// partial sums of <x, y> per slot (kRedBlocks per slot at `part`), then
+// partial sums of <x, y> per slot (red_blocks(n) per slot at `part`), then
 // out = sum (sqrt if asked)
 void dot_partials_batch(pm_ctx* c, int n_slots, const Batch& bt, int n, const double* x, const double* y,
                         double* part);
-void finish_sum_batch(pm_ctx* c, int n_slots, const Batch& bt, const double* part, double* out, bool take_sqrt);
+void finish_sum_batch(pm_ctx* c, int n_slots, const Batch& bt, int n, const double* part, double* out,
+                      bool take_sqrt);
 void nonactive_nonzero_batch(pm_ctx* c, int n_slots, const Batch& bt, const BlockMask& m, const double* x,
                              int* flag);
 

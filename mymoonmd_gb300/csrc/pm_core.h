@@ -125,6 +125,9 @@ struct pm_ctx {
   // launches of the sliced-ELL sweeps with programmatic stream serialization
   // (option "pdl": 0 off, 1 on)
   int pdl = 1;
+  // inside a multigrid cycle: small CSR launches with programmatic stream
+  // serialization too (the matrices were written before the cycle's first kernel)
+  bool in_cycle = false;
   // first Jacobi sweep from an exactly zero iterate as a diagonal scaling
   // (option "jacobi_zero_start"; same bits as the full sweep)
   bool jacobi_zero_start = true;
@@ -148,6 +151,14 @@ namespace pm {
 // the number of thread blocks used by every deterministic reduction
 constexpr int kRedBlocks = 304;  // 2 per SM on GB300
 constexpr int kRedThreads = 256;
+// Blocks of a reduction over n entries (their partial sums, in block order): two
+// entries per thread for short vectors. With all 304 blocks on 16,641 entries the
+// block trees' FP64 additions were most of the work (a batch of eight: 44 us for
+// the projections of one Arnoldi step).
+inline int red_blocks(int n) {
+  const int b = (n + 2 * kRedThreads - 1) / (2 * kRedThreads);
+  return b < 1 ? 1 : b < kRedBlocks ? b : kRedBlocks;
+}
 
 void ctx_init(pm_ctx* c, int device);
 void ctx_destroy(pm_ctx* c);

@@ -18,6 +18,25 @@ inline void launch_k(pm_ctx* c, void (*kern)(KArgs...), dim3 grid, dim3 block, s
   c->kernel_launches++;
 }
 
+// The same with programmatic stream serialization: the kernel waits (pdl_wait)
+// before it reads what the previous kernels write
+template <class... KArgs, class... Args>
+inline void launch_pdl(pm_ctx* c, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c->pdl >= 1 ? 1 : 0;
+  PM_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+  PM_CHECK_LAUNCH();
+  c->kernel_launches++;
+}
+
 // device CSR with optional FP32 copy of the values
 struct DevCsr {
   int n_rows = 0, n_cols = 0, n_active = 0;
@@ -84,6 +103,15 @@ void csr_apply(pm_ctx* c, const DevCsr& A, int epi, const double* x, double* y, 
                double alpha, int n_rows_override = -1);
 void csr_apply32(pm_ctx* c, const DevCsr& A, int epi, const float* x, float* y, const float* b,
                  float alpha, int n_rows_override = -1);
+// y := R x with the non-actives reset, x0 := w (y / d): the restriction and the
+// coarse level's first damped Jacobi sweep from a zero iterate
+void csr_restrict_zero(pm_ctx* c, const DevCsr& R, const double* x, double* y, const double* d, double w, double* x0);
+void csr_restrict_zero32(pm_ctx* c, const DevCsr& R, const float* x, float* y, const float* d, float w, float* x0);
+// start of a cycle: the level's right-hand side from the FP64 vector, and its
+// iterate: w (rhs / d) (zero, the first Jacobi sweep from zero), or zero with the
+// right-hand side's non-actives
+template <class T>
+void cycle_start(pm_ctx* c, int n, const BlockMask& m, const double* in, T* rhs, T* x, const T* d, T w, bool zero);
 
 // launch probe of SpMV-family kernels on matrices with `nnz` nonzeros
 void probe_reset(pm_ctx* c, int64_t nnz);
@@ -92,7 +120,7 @@ void probe_result(pm_ctx* c, int* count, double* total_ms, double* total_bytes);
 // BLAS-1 (deterministic fixed-tree reductions)
 void dot_partials(pm_ctx* c, int n, const double* x, const double* y, double* partials);
 double dot_host(pm_ctx* c, int n, const double* x, const double* y);  // synchronising
-void finish_sum(pm_ctx* c, const double* partials, double* out, bool take_sqrt);
+void finish_sum(pm_ctx* c, int n, const double* partials, double* out, bool take_sqrt);  // of dot_partials(n)
 void vcopy(pm_ctx* c, int n, const double* x, double* y);
 void vset(pm_ctx* c, int n, double* y, double v);
 void vscale(pm_ctx* c, int n, double* y, double a);
@@ -100,10 +128,6 @@ void vaxpy(pm_ctx* c, int n, double a, const double* x, double* y);  // y += a x
 void vaxpby(pm_ctx* c, int n, double a, const double* x, double b, double* y);  // y = a x + b y
 void vcvt_d2f(pm_ctx* c, int n, const double* x, float* y);
 void vcvt_f2d(pm_ctx* c, int n, const float* x, double* y);
-void vcopy32(pm_ctx* c, int n, const float* x, float* y);
-// sol := 0 on active rows, rhs on non-active rows (Multigrid::cycle start)
-void init_solution(pm_ctx* c, int n, const BlockMask& m, const double* rhs, double* sol);
-void init_solution32(pm_ctx* c, int n, const BlockMask& m, const float* rhs, float* sol);
 // x := w (b / d), the damped Jacobi sweep from x = 0
 void jacobi_from_zero(pm_ctx* c, int n, const double* b, const double* d, double w, double* x);
 void jacobi_from_zero32(pm_ctx* c, int n, const float* b, const float* d, float w, float* x);

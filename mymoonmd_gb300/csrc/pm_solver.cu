@@ -396,11 +396,16 @@ void Multigrid::defect(pm_ctx* c, int l) {
   else csr_apply(c, lv.A->csr, EPI_DEFECT, lv.cur, lv.defect.p, lv.rhs.p, 1.0);
 }
 
-void Multigrid::restrict_to(pm_ctx* c, int l) {
+void Multigrid::restrict_to(pm_ctx* c, int l, bool sweep) {
   MGLevel& fine = levels[l];
   MGLevel& crs = levels[l - 1];
   // DefectRestriction followed by ResetNonActive of the coarse rhs
-  if (mixed) csr_apply32(c, crs.R, EPI_RESTRICT, fine.defect32.p, crs.rhs32.p, nullptr, 1.0f);
+  const DevCsr& A = crs.A->csr;
+  if (sweep && mixed)
+    csr_restrict_zero32(c, crs.R, fine.defect32.p, crs.rhs32.p, A.diag32.p, float(jacobi_damp), crs.cur32);
+  else if (sweep)
+    csr_restrict_zero(c, crs.R, fine.defect.p, crs.rhs.p, A.diag.p, jacobi_damp, crs.cur);
+  else if (mixed) csr_apply32(c, crs.R, EPI_RESTRICT, fine.defect32.p, crs.rhs32.p, nullptr, 1.0f);
   else csr_apply(c, crs.R, EPI_RESTRICT, fine.defect.p, crs.rhs.p, nullptr, 1.0);
 }
 
@@ -429,19 +434,27 @@ void Multigrid::apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonact
     lv.cur32 = lv.sol32.p;
     lv.oth32 = lv.alt32.p;
   }
-  // set_finest_rhs / set_finest_sol; cycle(): solution := 0, copy_nonactive(rhs)
-  if (mixed) {
-    vcvt_d2f(c, nf, rhs, top.rhs32.p);
-    init_solution32(c, nf, top.A->csr.mask, top.rhs32.p, top.cur32);
-  } else {
-    vcopy(c, nf, rhs, top.rhs.p);
-    init_solution(c, nf, top.A->csr.mask, top.rhs.p, top.cur);
-  }
+  // set_finest_rhs / set_finest_sol; cycle(): solution := 0, copy_nonactive(rhs);
+  // with zero non-actives the first Jacobi sweep comes with it
+  const bool jz = c->jacobi_zero_start && n_pre >= 1;  // first Jacobi sweeps from zero are fused
+  const bool top_swept = finest > 0 && jz && rhs_nonactive_zero && top.smoother == SM_JACOBI;
+  if (mixed)
+    cycle_start<float>(c, nf, top.A->csr.mask, rhs, top.rhs32.p, top.cur32, top.A->csr.diag32.p, float(jacobi_damp),
+                       top_swept);
+  else
+    cycle_start<double>(c, nf, top.A->csr.mask, rhs, top.rhs.p, top.cur, top.A->csr.diag.p, jacobi_damp, top_swept);
+  struct InCycle {
+    pm_ctx* c;
+    explicit InCycle(pm_ctx* c_) : c(c_) { c->in_cycle = true; }
+    ~InCycle() { c->in_cycle = false; }
+  } in_cycle(c);
   // levels whose iterate is exactly zero now: the finest one when its rhs has
   // zero non-actives (init_solution copies them), the coarser ones after their
   // reset below (their rhs has its non-actives reset by the restriction)
-  std::vector<char> zero(L, 0);
+  // swept: the level's first sweep from zero has been done with its right-hand side
+  std::vector<char> zero(L, 0), swept(L, 0);
   zero[finest] = rhs_nonactive_zero ? 1 : 0;
+  swept[finest] = top_swept ? 1 : 0;
   const int n_steps = int(control.size()) - 1;
   int level = finest;
   for (int step = 1; step <= n_steps && level >= 0; ++step) {
@@ -463,7 +476,8 @@ void Multigrid::apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonact
       for (int i = 0; i < n_post; ++i) smooth(c, level);
     if (down) {
       for (int i = 0; i < n_pre; ++i) {
-        if (i == 0 && zero[level]) smooth_from_zero(c, level);
+        if (i == 0 && swept[level]) swept[level] = 0;
+        else if (i == 0 && zero[level]) smooth_from_zero(c, level);
         else smooth(c, level);
         zero[level] = 0;
       }
@@ -480,7 +494,8 @@ void Multigrid::apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonact
         else PM_CUDA(cudaMemsetAsync(crs.cur, 0, sizeof(double) * nc, c->stream));
       }
       zero[level - 1] = 1;
-      restrict_to(c, level);
+      swept[level - 1] = jz && level - 1 > 0 && crs.smoother == SM_JACOBI;
+      restrict_to(c, level, swept[level - 1] != 0);
       level -= 1;
     } else if (up) {
       prolongate_from(c, level);
@@ -498,10 +513,10 @@ static int grid_blocks_for(int n) { return std::max(1, std::min((n + 255) / 256,
 
 // ------------------------------------------------------ FGMRES kernels -----
 // every block sums the partials of the previous reduction in the same order
-__device__ __forceinline__ double sum_partials(const double* __restrict__ part, double* sh) {
+__device__ __forceinline__ double sum_partials(const double* __restrict__ part, double* sh, int np) {
   const int t = threadIdx.x;
   double s = 0.0;
-  for (int i = t; i < kRedBlocks; i += blockDim.x) s += part[i];
+  for (int i = t; i < np; i += blockDim.x) s += part[i];
   sh[t] = s;
   __syncthreads();
   for (int k = blockDim.x / 2; k > 0; k >>= 1) {
@@ -531,7 +546,7 @@ __global__ void __launch_bounds__(256) k_fg_mgs(int n, int ldh, int k, int i, do
                                                 const double* __restrict__ part_in,
                                                 double* __restrict__ part_out, double* __restrict__ H) {
   __shared__ double sh[256];
-  const double h = sum_partials(part_in, sh);
+  const double h = sum_partials(part_in, sh, gridDim.x);  // launched with as many blocks as partials
   if (blockIdx.x == 0 && threadIdx.x == 0) H[k + (size_t)ldh * i] = h;
   double acc = 0.0;
   const double mh = -h;
@@ -551,7 +566,7 @@ __device__ __forceinline__ void fg_normalize_body(int n, int ldh, int i, const d
                                                       double* __restrict__ H, int* __restrict__ flag) {
   pdl_enter();
   __shared__ double sh[256];
-  const double hn = sqrt(sum_partials(part_in, sh));
+  const double hn = sqrt(sum_partials(part_in, sh, gridDim.x));
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     H[(i + 1) + (size_t)ldh * i] = hn;
     if (hn == 0.0) flag[0] = 1;
@@ -573,7 +588,7 @@ __device__ __forceinline__ void fg_start_body(int n, int m, const double* __rest
                                                   const double* __restrict__ part_in,
                                                   double* __restrict__ s, double* __restrict__ beta_out) {
   __shared__ double sh[256];
-  const double beta = sqrt(sum_partials(part_in, sh));
+  const double beta = sqrt(sum_partials(part_in, sh, gridDim.x));
   if (blockIdx.x == 0) {
     for (int k = threadIdx.x; k <= m; k += blockDim.x) s[k] = (k == 0) ? beta : 0.0;
     if (threadIdx.x == 0) *beta_out = beta;
@@ -631,7 +646,7 @@ __global__ void __launch_bounds__(256) k_multidot(int n, int nk, const double* _
 // guard set (second pass skipped): h[k] = 0 and H(k, col) = hsum[k]
 __device__ __forceinline__ void reduce_proj_body(const double* __restrict__ part, double* __restrict__ h,
                                                      const double* __restrict__ hsum, double* __restrict__ H,
-                                                     int ldh, int col, const int* __restrict__ guard) {
+                                                     int ldh, int col, int np, const int* __restrict__ guard) {
   pdl_enter();
   __shared__ double sh[256];
   const int k = blockIdx.x;
@@ -642,7 +657,7 @@ __device__ __forceinline__ void reduce_proj_body(const double* __restrict__ part
     }
     return;
   }
-  const double s = sum_partials(part + (size_t)k * kRedBlocks, sh);
+  const double s = sum_partials(part + (size_t)k * kRedBlocks, sh, np);
   if (threadIdx.x == 0) {
     h[k] = s;
     if (hsum) H[k + (size_t)ldh * col] = hsum[k] + s;
@@ -650,8 +665,8 @@ __device__ __forceinline__ void reduce_proj_body(const double* __restrict__ part
 }
 __global__ void __launch_bounds__(256) k_reduce_proj(const double* __restrict__ part, double* __restrict__ h,
                                                      const double* __restrict__ hsum, double* __restrict__ H,
-                                                     int ldh, int col, const int* __restrict__ guard) {
-  reduce_proj_body(part, h, hsum, H, ldh, col, guard);
+                                                     int ldh, int col, int np, const int* __restrict__ guard) {
+  reduce_proj_body(part, h, hsum, H, ldh, col, np, guard);
 }
 
 // r -= sum_k h[k] V_k, subtracted in k order
@@ -855,10 +870,10 @@ __global__ void __launch_bounds__(256, 2) k_cgs_update_norm(int n, int nk, doubl
 
 // DGKS test after the first classical Gram-Schmidt pass: the second pass is
 // needed only if |r after| < |r before| / sqrt(2); flag = 1 skips it
-__global__ void k_cgs_decide(const double* __restrict__ part_after, const double* __restrict__ rr_before,
+__global__ void k_cgs_decide(const double* __restrict__ part_after, int np, const double* __restrict__ rr_before,
                              int* __restrict__ flag) {
   __shared__ double sh[256];
-  const double after = sum_partials(part_after, sh);
+  const double after = sum_partials(part_after, sh, np);
   if (threadIdx.x == 0) *flag = (after >= 0.5 * rr_before[0]) ? 1 : 0;
 }
 
@@ -884,16 +899,38 @@ __device__ void app_rot(double& dx, double& dy, double cs, double sn) {
   dx = t;
 }
 
+// one warp: the column and the rotations come to shared memory in one round of
+// loads (read one by one from L2, ten rotations took 7 us)
 __device__ __forceinline__ void fg_givens_body(int ldh, int i, double* __restrict__ H, double* __restrict__ cs,
                             double* __restrict__ sn, double* __restrict__ s, double* __restrict__ resid) {
   pdl_enter();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double* col = H + (size_t)ldh * i;
-  for (int k = 0; k < i; ++k) app_rot(col[k], col[k + 1], cs[k], sn[k]);
-  gen_rot(col[i], col[i + 1], cs[i], sn[i]);
-  app_rot(col[i], col[i + 1], cs[i], sn[i]);
-  app_rot(s[i], s[i + 1], cs[i], sn[i]);
-  *resid = fabs(s[i + 1]);
+  __shared__ double col[64], c[64], d[64];  // i < 60
+  const int t = threadIdx.x;
+  if (t >= 32 || blockIdx.x != 0) return;
+  double* hc = H + (size_t)ldh * i;
+  for (int k = t; k <= i + 1; k += 32) {
+    col[k] = hc[k];
+    if (k < i) {
+      c[k] = cs[k];
+      d[k] = sn[k];
+    }
+  }
+  double s0 = s[i], s1 = s[i + 1];
+  __syncwarp();
+  if (t == 0) {
+    for (int k = 0; k < i; ++k) app_rot(col[k], col[k + 1], c[k], d[k]);
+    double cc, dd;
+    gen_rot(col[i], col[i + 1], cc, dd);
+    app_rot(col[i], col[i + 1], cc, dd);
+    app_rot(s0, s1, cc, dd);
+    cs[i] = cc;
+    sn[i] = dd;
+    s[i] = s0;
+    s[i + 1] = s1;
+    *resid = fabs(s1);
+  }
+  __syncwarp();
+  for (int k = t; k <= i + 1; k += 32) hc[k] = col[k];
 }
 __global__ void k_fg_givens(int ldh, int i, double* __restrict__ H, double* __restrict__ cs,
                             double* __restrict__ sn, double* __restrict__ s, double* __restrict__ resid) {
@@ -901,14 +938,36 @@ __global__ void k_fg_givens(int ldh, int i, double* __restrict__ H, double* __re
 }
 
 // Update (src/Solver/Iteration_gmres.C:152): back-solve H y = s
+// one warp, entries lane and lane + 32 of y; the next column is loaded before
+// the current one is used (one thread reading H entry by entry took 62 us for 27
+// columns)
 __device__ __forceinline__ void fg_backsolve_body(int ldh, int k, const double* __restrict__ H,
                                const double* __restrict__ s, double* __restrict__ y) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int i = 0; i <= k; ++i) y[i] = s[i];
+  const int t = threadIdx.x;
+  if (t >= 32 || blockIdx.x != 0) return;
+  double y0 = t <= k ? s[t] : 0.0, y1 = t + 32 <= k ? s[t + 32] : 0.0;
+  auto col = [&](int i, double& a, double& b, double& d) {
+    const double* h = H + (size_t)ldh * i;
+    a = t < i ? h[t] : 0.0;
+    b = t + 32 < i ? h[t + 32] : 0.0;
+    d = h[i];
+  };
+  double a, b, d;
+  col(k, a, b, d);
   for (int i = k; i >= 0; --i) {
-    y[i] /= H[i + (size_t)ldh * i];
-    for (int j = i - 1; j >= 0; --j) y[j] -= H[j + (size_t)ldh * i] * y[i];
+    double an = 0.0, bn = 0.0, dn = 1.0;
+    if (i > 0) col(i - 1, an, bn, dn);
+    const double yi = __shfl_sync(0xffffffffu, i < 32 ? y0 : y1, i & 31) / d;
+    if (t == i) y0 = yi;
+    if (t + 32 == i) y1 = yi;
+    if (t < i) y0 -= a * yi;
+    if (t + 32 < i) y1 -= b * yi;
+    a = an;
+    b = bn;
+    d = dn;
   }
+  if (t <= k) y[t] = y0;
+  if (t + 32 <= k) y[t + 32] = y1;
 }
 __global__ void k_fg_backsolve(int ldh, int k, const double* __restrict__ H,
                                const double* __restrict__ s, double* __restrict__ y) {
@@ -954,10 +1013,10 @@ __global__ void __launch_bounds__(256, 2) kb_mdot(int n, int nk, const double* _
 }
 __global__ void __launch_bounds__(256) kb_reduce_proj(const double* __restrict__ part, double* __restrict__ h,
                                                       const double* __restrict__ hsum, double* __restrict__ H, int ldh,
-                                                      int col, Batch bt) {
+                                                      int col, int np, Batch bt) {
   if (!bt.on[blockIdx.y]) return;
   PM_SLOT(part); PM_SLOT(h); PM_SLOT(hsum); PM_SLOT(H);
-  reduce_proj_body(part, h, hsum, H, ldh, col, nullptr);
+  reduce_proj_body(part, h, hsum, H, ldh, col, np, nullptr);
 }
 template <int NK>
 __global__ void __launch_bounds__(256, 2) kb_cgs_update_mdot(int n, int nk, double* __restrict__ r,
@@ -1005,7 +1064,7 @@ __global__ void __launch_bounds__(256) kb_fg_combine(int n, int k, const double*
 
 void fg_start_batch(pm_ctx* c, int ns, const Batch& bt, int n, int m, const double* r, double* v0,
                     const double* part, double* s, double* beta_out) {
-  kb_fg_start<<<dim3(kRedBlocks, unsigned(ns)), 256, 0, c->stream>>>(n, m, r, v0, part, s, beta_out, bt);
+  kb_fg_start<<<dim3(unsigned(red_blocks(n)), unsigned(ns)), 256, 0, c->stream>>>(n, m, r, v0, part, s, beta_out, bt);
   PM_CHECK_LAUNCH();
   c->kernel_launches++;
 }
@@ -1015,13 +1074,14 @@ void fg_cgs2_batch(pm_ctx* c, int ns, const Batch& bt, int n, int i, int ldh, do
                    double* cgs_part, double* h1, double* h2, double* H, double* part_norm) {
   const int nk = i + 1;
   if (nk > kCgsFused) throw Error(PM_E_UNSUPPORTED, "batched FGMRES needs gmres_restart <= 32");
-  const dim3 rb = dim3(kRedBlocks, unsigned(ns)), pk = dim3(unsigned(nk), unsigned(ns)), t256 = dim3(256);
+  const int np = red_blocks(n);
+  const dim3 rb = dim3(unsigned(np), unsigned(ns)), pk = dim3(unsigned(nk), unsigned(ns)), t256 = dim3(256);
   if (nk <= 16) kb_mdot<16><<<rb, t256, 0, c->stream>>>(n, nk, r, V, ld, cgs_part, bt);
   else kb_mdot<kCgsFused><<<rb, t256, 0, c->stream>>>(n, nk, r, V, ld, cgs_part, bt);
-  kb_reduce_proj<<<pk, t256, 0, c->stream>>>(cgs_part, h1, nullptr, H, ldh, i, bt);
+  kb_reduce_proj<<<pk, t256, 0, c->stream>>>(cgs_part, h1, nullptr, H, ldh, i, np, bt);
   if (nk <= 16) kb_cgs_update_mdot<16><<<rb, t256, 0, c->stream>>>(n, nk, r, V, ld, h1, cgs_part, bt);
   else kb_cgs_update_mdot<kCgsFused><<<rb, t256, 0, c->stream>>>(n, nk, r, V, ld, h1, cgs_part, bt);
-  kb_reduce_proj<<<pk, t256, 0, c->stream>>>(cgs_part, h2, h1, H, ldh, i, bt);
+  kb_reduce_proj<<<pk, t256, 0, c->stream>>>(cgs_part, h2, h1, H, ldh, i, np, bt);
   kb_cgs_update_norm<<<rb, t256, 0, c->stream>>>(n, nk, r, V, ld, h2, part_norm, bt);
   PM_CHECK_LAUNCH();
   c->kernel_launches += 5;
@@ -1029,7 +1089,7 @@ void fg_cgs2_batch(pm_ctx* c, int ns, const Batch& bt, int n, int i, int ldh, do
 
 void fg_normalize_batch(pm_ctx* c, int ns, const Batch& bt, int n, int ldh, int i, const double* r, double* v,
                         const double* part, double* H, int* flag) {
-  kb_fg_normalize<<<dim3(kRedBlocks, unsigned(ns)), 256, 0, c->stream>>>(n, ldh, i, r, v, part, H, flag, bt);
+  kb_fg_normalize<<<dim3(unsigned(red_blocks(n)), unsigned(ns)), 256, 0, c->stream>>>(n, ldh, i, r, v, part, H, flag, bt);
   PM_CHECK_LAUNCH();
   c->kernel_launches++;
 }
@@ -1199,7 +1259,7 @@ void pm_solver::fgmres(const double* rhs, double* sol) {
   PM_CUDA(cudaMemsetAsync(flags.p + 2, 0, sizeof(int), c->stream));
   nonactive_nonzero(c, M.mask, r, flags.p + 2);
   dot_partials(c, n, r, r, partA);
-  finish_sum(c, partA, dres, true);
+  finish_sum(c, n, partA, dres, true);
   PM_CUDA(cudaMemcpyAsync(c->host_scalars, dres, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   PM_CUDA(cudaMemcpyAsync(reinterpret_cast<int*>(c->host_scalars + 2), flags.p + 2, sizeof(int),
                           cudaMemcpyDeviceToHost, c->stream));
@@ -1216,7 +1276,7 @@ void pm_solver::fgmres(const double* rhs, double* sol) {
   }
   if (converged(resid, 0)) return;
 
-  const int grid = kRedBlocks;
+  const int grid = red_blocks(n);
   const bool cgs_cond = gram_schmidt == "cgs2_cond";
   const bool cgs2 = gram_schmidt == "cgs2" || cgs_cond;
   unsigned j = 1;
@@ -1241,17 +1301,17 @@ void pm_solver::fgmres(const double* rhs, double* sol) {
           // two classical Gram-Schmidt passes in three sweeps over the basis;
           // H(:,i) = h1 + h2, |r|^2 partials into partA
           const int nk = i + 1;
-          const dim3 rb(kRedBlocks), t256(256);
+          const dim3 rb(grid), t256(256);
           const double* Vc = V;
           const double* nul = nullptr;
           const int* inul = nullptr;
           if (nk <= 16) launch_k(c, k_mdot<16>, rb, t256, 0, n, nk, (const double*)r, Vc, ld, cgs_part);
           else launch_k(c, k_mdot<kCgsFused>, rb, t256, 0, n, nk, (const double*)r, Vc, ld, cgs_part);
-          launch_k(c, k_reduce_proj, dim3(nk), t256, 0, (const double*)cgs_part, h1, nul, H, ldh, i, inul);
+          launch_k(c, k_reduce_proj, dim3(nk), t256, 0, (const double*)cgs_part, h1, nul, H, ldh, i, grid, inul);
           if (nk <= 16) launch_k(c, k_cgs_update_mdot<16>, rb, t256, 0, n, nk, r, Vc, ld, (const double*)h1, cgs_part);
           else launch_k(c, k_cgs_update_mdot<kCgsFused>, rb, t256, 0, n, nk, r, Vc, ld, (const double*)h1, cgs_part);
           launch_k(c, k_reduce_proj, dim3(nk), t256, 0, (const double*)cgs_part, h2, (const double*)h1, H, ldh, i,
-                     inul);
+                   grid, inul);
           launch_k(c, k_cgs_update_norm, rb, t256, 0, n, nk, r, Vc, ld, (const double*)h2, partA);
         } else if (cgs2) {
           // two passes of classical Gram-Schmidt; H(:,i) = h1 + h2. With the
@@ -1259,18 +1319,18 @@ void pm_solver::fgmres(const double* rhs, double* sol) {
           // more than a factor 1/sqrt(2) of the norm (decided on the device)
           const int nk = i + 1;
           const int ub = grid_blocks_for(n);
-          k_multidot<8><<<kRedBlocks, 256, 0, c->stream>>>(n, nk, r, V, ld, cgs_part, cgs_cond ? 1 : 0, nullptr);
-          k_reduce_proj<<<nk + (cgs_cond ? 1 : 0), 256, 0, c->stream>>>(cgs_part, h1, nullptr, H, ldh, i, nullptr);
+          k_multidot<8><<<grid, 256, 0, c->stream>>>(n, nk, r, V, ld, cgs_part, cgs_cond ? 1 : 0, nullptr);
+          k_reduce_proj<<<nk + (cgs_cond ? 1 : 0), 256, 0, c->stream>>>(cgs_part, h1, nullptr, H, ldh, i, grid, nullptr);
           k_cgs_update<<<ub, 256, 0, c->stream>>>(n, nk, r, V, ld, h1, nullptr);
           const int* skip = nullptr;
           if (cgs_cond) {
             dot_partials(c, n, r, r, partB);
-            k_cgs_decide<<<1, 256, 0, c->stream>>>(partB, h1 + nk, flags.p + 1);
+            k_cgs_decide<<<1, 256, 0, c->stream>>>(partB, grid, h1 + nk, flags.p + 1);
             c->kernel_launches++;
             skip = flags.p + 1;
           }
-          k_multidot<8><<<kRedBlocks, 256, 0, c->stream>>>(n, nk, r, V, ld, cgs_part, 0, skip);
-          k_reduce_proj<<<nk, 256, 0, c->stream>>>(cgs_part, h2, h1, H, ldh, i, skip);
+          k_multidot<8><<<grid, 256, 0, c->stream>>>(n, nk, r, V, ld, cgs_part, 0, skip);
+          k_reduce_proj<<<nk, 256, 0, c->stream>>>(cgs_part, h2, h1, H, ldh, i, grid, skip);
           k_cgs_update<<<ub, 256, 0, c->stream>>>(n, nk, r, V, ld, h2, skip);
           PM_CHECK_LAUNCH();
           c->kernel_launches += 6;
@@ -1358,7 +1418,7 @@ void pm_solver::fgmres(const double* rhs, double* sol) {
       // the solution is unchanged since the start of this cycle
       csr_apply(c, M, EPI_DEFECT, sol, r, rhs, 1.0);
       dot_partials(c, n, r, r, partA);
-      finish_sum(c, partA, dres, true);
+      finish_sum(c, n, partA, dres, true);
       PM_CUDA(cudaMemcpyAsync(c->host_scalars, dres, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
       PM_CUDA(cudaStreamSynchronize(c->stream));
       resid = c->host_scalars[0];

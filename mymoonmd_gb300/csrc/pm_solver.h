@@ -93,7 +93,8 @@ struct Multigrid {
   // +0); other smoothers sweep as usual
   void smooth_from_zero(pm_ctx* c, int l);
   void defect(pm_ctx* c, int l);
-  void restrict_to(pm_ctx* c, int l);  // from l to l-1
+  // from l to l-1; sweep: with the first Jacobi sweep of l-1 from zero
+  void restrict_to(pm_ctx* c, int l, bool sweep);
   void prolongate_from(pm_ctx* c, int l);  // from l to l+1
   void coarse_solve(pm_ctx* c);
   // switch the cycle between FP32 and FP64 (FGMRES is flexible, so the

@@ -21,7 +21,12 @@
 
 namespace pm {
 
-enum Epi { EPI_AXPY = 0, EPI_SET = 1, EPI_DEFECT = 2, EPI_JACOBI = 3, EPI_RESTRICT = 4, EPI_PROLONG = 5 };
+// RESTRICT_ZERO is RESTRICT followed by the damped Jacobi sweep of the coarse
+// level from a zero iterate, x0_i = fma(w, y_i / d_i, 0) with w = alpha; x0 comes in
+// the place of b
+enum Epi {
+  EPI_AXPY = 0, EPI_SET = 1, EPI_DEFECT = 2, EPI_JACOBI = 3, EPI_RESTRICT = 4, EPI_PROLONG = 5, EPI_RESTRICT_ZERO = 6
+};
 
 // Up to four contiguous blocks [start, end) of a block vector; rows in
 // [active_end, end) of each block are non-active.
@@ -60,43 +65,34 @@ __device__ __forceinline__ void pdl_enter() {
   pdl_wait();
 }
 
+template <class T>
+__device__ __forceinline__ T fmadd(T a, T b, T c);
+template <>
+__device__ __forceinline__ float fmadd<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+template <>
+__device__ __forceinline__ double fmadd<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
+
 // G lanes per row, U entries per lane per chunk: a lane first issues its U
 // value and U column loads, then its U gathers of x, then the U products, so
-// that every lane keeps U independent DRAM requests in flight.
+// that every lane keeps U independent DRAM requests in flight. Launched with
+// programmatic stream serialization (small launches inside a multigrid cycle), the
+// row bounds and the first chunk are loaded before the wait for the previous
+// kernel.
 template <class TV, class TX, class TA, int G, int U, int EPI>
 __device__ __forceinline__ void
 csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ cols,
          const TV* __restrict__ vals, const TX* __restrict__ x, TX* __restrict__ y,
          const TX* __restrict__ b, const TX* __restrict__ diag, const TX* __restrict__ xold,
          TA alpha, const BlockMask& mask, int bx, int gx) {
-  pdl_enter();
-  if (guarded(mask.guard)) {  // uniform for the whole grid
-    // a skipped Jacobi sweep leaves the iterate as it is (the caller swaps
-    // the two iterate buffers after every sweep)
-    if (EPI == EPI_JACOBI)
-      for (int i = bx * blockDim.x + threadIdx.x; i < n_rows; i += gx * blockDim.x) y[i] = xold[i];
-    return;
-  }
+  pdl_trigger();
   const int lane = threadIdx.x & (G - 1);
   const int row = (bx * blockDim.x + threadIdx.x) / G;
   const bool valid = row < n_rows;  // whole groups share a row: no early exit before the shuffles
   const int beg = valid ? __ldg(row_ptr + row) : 0;
   const int end = valid ? __ldg(row_ptr + row + 1) : 0;
-  // the epilogue's per-row operands are loaded before the row walk, so their
-  // latency overlaps with it instead of following the reduction
-  TX pre_b = TX(0), pre_d = TX(1), pre_x = TX(0), pre_y = TX(0);
-  if (valid && lane == 0) {
-    if constexpr (EPI == EPI_AXPY || EPI == EPI_PROLONG) pre_y = y[row];
-    if constexpr (EPI == EPI_DEFECT || EPI == EPI_JACOBI) pre_b = __ldg(b + row);
-    if constexpr (EPI == EPI_JACOBI) {
-      pre_d = __ldg(diag + row);
-      pre_x = __ldg(xold + row);
-    }
-  }
-  TA s = TA(0);
-  for (int base = beg; base < end; base += G * U) {
-    TV v[U];
-    int c[U];
+  TV v[U];
+  int c[U];
+  auto load = [&](int base) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = base + u * G + lane;
@@ -108,11 +104,33 @@ csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ co
         c[u] = 0;  // x[0] exists whenever the row has entries
       }
     }
+  };
+  if (beg < end) load(beg);
+  pdl_wait();
+  if (guarded(mask.guard)) {  // uniform for the whole grid
+    // a skipped Jacobi sweep leaves the iterate as it is (the caller swaps
+    // the two iterate buffers after every sweep)
+    if (EPI == EPI_JACOBI)
+      for (int i = bx * blockDim.x + threadIdx.x; i < n_rows; i += gx * blockDim.x) y[i] = xold[i];
+    return;
+  }
+  // the epilogue's per-row operands are loaded before the row walk, so their
+  // latency overlaps with it instead of following the reduction
+  TX pre_b = TX(0), pre_d = TX(1), pre_x = TX(0), pre_y = TX(0);
+  if (valid && lane == 0) {
+    if constexpr (EPI == EPI_AXPY || EPI == EPI_PROLONG) pre_y = y[row];
+    if constexpr (EPI == EPI_DEFECT || EPI == EPI_JACOBI) pre_b = __ldg(b + row);
+    if constexpr (EPI == EPI_JACOBI || EPI == EPI_RESTRICT_ZERO) pre_d = __ldg(diag + row);
+    if constexpr (EPI == EPI_JACOBI) pre_x = __ldg(xold + row);
+  }
+  TA s = TA(0);
+  for (int base = beg; base < end; base += G * U) {
     TX xv[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c[u]);
 #pragma unroll
     for (int u = 0; u < U; ++u) s += TA(v[u]) * TA(xv[u]);
+    if (base + G * U < end) load(base + G * U);
   }
 #pragma unroll
   for (int off = G / 2; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off, G);
@@ -129,6 +147,10 @@ csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ co
     y[row] = TX(TA(pre_x) + alpha * d);
   } else if constexpr (EPI == EPI_RESTRICT) {
     y[row] = row_is_active(mask, row) ? TX(s) : TX(0);
+  } else if constexpr (EPI == EPI_RESTRICT_ZERO) {
+    const TX r = row_is_active(mask, row) ? TX(s) : TX(0);
+    y[row] = r;
+    const_cast<TX*>(b)[row] = fmadd(TX(alpha), (r - TX(0)) / pre_d, TX(0));
   } else if constexpr (EPI == EPI_PROLONG) {
     if (row_is_active(mask, row)) y[row] = TX(TA(pre_y) + alpha * s);
   }
@@ -217,6 +239,10 @@ csr_stream_kernel(const int* __restrict__ rblock, const int* __restrict__ row_pt
         y[row] = TX(TA(x[row]) + alpha * d);
       } else if constexpr (EPI == EPI_RESTRICT) {
         y[row] = row_is_active(mask, row) ? TX(sum) : TX(0);
+      } else if constexpr (EPI == EPI_RESTRICT_ZERO) {
+        const TX r = row_is_active(mask, row) ? TX(sum) : TX(0);
+        y[row] = r;
+        const_cast<TX*>(b)[row] = fmadd(TX(alpha), (r - TX(0)) / diag[row], TX(0));
       } else if constexpr (EPI == EPI_PROLONG) {
         if (row_is_active(mask, row)) y[row] = TX(TA(y[row]) + alpha * sum);
       }
@@ -241,13 +267,6 @@ csr_stream_kernel(const int* __restrict__ rblock, const int* __restrict__ row_pt
 // serialization, a sweep loads its permutation, slice offsets and (PIPE) first
 // U steps while the previous kernel finishes.
 constexpr int kSellWindow = 1024;
-
-template <class T>
-__device__ __forceinline__ T fmadd(T a, T b, T c);
-template <>
-__device__ __forceinline__ float fmadd<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-template <>
-__device__ __forceinline__ double fmadd<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 template <class T, int L, int U, bool PIPE, int EPI>
 __device__ __forceinline__ void
@@ -287,10 +306,8 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
   if (row >= 0 && sub == 0) {
     if constexpr (EPI == EPI_AXPY || EPI == EPI_PROLONG) pre_y = y[row];
     if constexpr (EPI == EPI_DEFECT || EPI == EPI_JACOBI) pre_b = __ldg(b + row);
-    if constexpr (EPI == EPI_JACOBI) {
-      pre_d = __ldg(diag + row);
-      pre_x = __ldg(x + row);
-    }
+    if constexpr (EPI == EPI_JACOBI || EPI == EPI_RESTRICT_ZERO) pre_d = __ldg(diag + row);
+    if constexpr (EPI == EPI_JACOBI) pre_x = __ldg(x + row);
   }
   T acc = T(0);
   if constexpr (!PIPE) {
@@ -341,6 +358,10 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
     y[row] = pre_x + alpha * d;
   } else if constexpr (EPI == EPI_RESTRICT) {
     y[row] = row_is_active(mask, row) ? acc : T(0);
+  } else if constexpr (EPI == EPI_RESTRICT_ZERO) {
+    const T r = row_is_active(mask, row) ? acc : T(0);
+    y[row] = r;
+    const_cast<T*>(b)[row] = fmadd(alpha, (r - T(0)) / pre_d, T(0));
   } else if constexpr (EPI == EPI_PROLONG) {
     if (row_is_active(mask, row)) y[row] = pre_y + alpha * acc;
   }
