@@ -68,14 +68,17 @@ void DevCsr::upload(pm_ctx* c, int nr, int nc, int na, const int* rp, const int*
     if (nnz) PM_CUDA(cudaMemsetAsync(vals.p, 0, vals.bytes(), c->stream));
   }
   drop_sell();  // a new structure: no sliced layout yet
-  // measured on GB300 (3D Q2, 15.8 M and 54.5 M nonzeros): four lanes per row
-  // with eight loads in flight per lane is the fastest launch shape for both
-  // FP64 and FP32 values; short rows take four loads per lane
-  // FP64: four lanes x eight loads (the FP64 pipe is the limit); FP32: eight
-  // lanes x sixteen loads in flight (3.9 TB/s vs 3.4 TB/s at four x eight)
+  // measured on GB300. FP64: an instruction costs a sub-core about 75 clocks, so
+  // short rows (at most 16 entries on average) take two lanes: half as many
+  // additions and Jacobi divisions per row as with four. FP64 cycle of 2D Q1 in us,
+  // four lanes / two / one: 128^2 76 / 72 / 78, 256^2 121 / 105 / 103, 512^2
+  // 298 / 224 / 221, 1024^2 1315 / 1008 / 965; 2D Q2 128^2 154 / 128 / 144,
+  // 512^2 1649 / 1202 / 1261. Long rows: four lanes x eight loads. FP32: eight
+  // lanes x sixteen loads in flight (3.9 TB/s vs 3.4 TB/s at four x eight on
+  // 15.8 M and 54.5 M nonzeros), short rows four x four
   const double avg = nr ? double(nnz) / nr : 1.0;
-  lanes = 4;
-  unroll = avg > 16.0 ? 8 : 4;
+  lanes = avg > 16.0 ? 4 : 2;
+  unroll = 8;
   lanes32 = avg > 16.0 ? 8 : 4;
   unroll32 = avg > 16.0 ? 16 : 4;
   stream = false;
@@ -449,6 +452,12 @@ static void launch_sell_shape(pm_ctx* c, const DevCsr& A, int epi, const T* x, T
   }
 }
 
+// FP64 shape 441 on matrices of few slices: eight steps in flight instead of four
+// (the sums are the same). At most 128 slices per SM, FP64 cycle of 3D Q2 in us,
+// four / eight: 16^3 (36 slices per SM in the finest sweep) 129 / 105, 24^3 (97)
+// 235 / 220, 28^3 (152) 263 / 271, 32^3 (226) 378 / 378 with the SpMV 39.2 / 42.8
+static bool sell_deep(const pm_ctx* c, long long n_slices) { return n_slices <= 128ll * c->num_sms; }
+
 static void launch_sell(pm_ctx* c, const DevCsr& A, int epi, const float* x, float* y, const float* b,
                         const float* d, float alpha) {
   BlockMask mg = A.mask;
@@ -463,7 +472,9 @@ static void launch_sell(pm_ctx* c, const DevCsr& A, int epi, const float* x, flo
     case 440: launch_sell_shape<float, 4, 4, false>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 441: launch_sell_shape<float, 4, 4, true>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 480: launch_sell_shape<float, 4, 8, false>(c, A, epi, x, y, b, d, alpha, mg); break;
-    case 481: launch_sell_shape<float, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg); break;
+    // sixteen steps in flight: mixed cycle of 3D Q2 in us, eight / sixteen: 8^3
+    // 41.9 / 38.3, 16^3 63.9 / 57.5, 24^3 122.5 / 115.4, 32^3 194 / 190
+    case 481: launch_sell_shape<float, 4, 16, true>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 840: launch_sell_shape<float, 8, 4, false>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 841: launch_sell_shape<float, 8, 4, true>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 881: launch_sell_shape<float, 8, 8, true>(c, A, epi, x, y, b, d, alpha, mg); break;
@@ -478,7 +489,10 @@ static void launch_sell64(pm_ctx* c, const DevCsr& A, int epi, const double* x, 
   BlockMask mg = A.mask;
   mg.guard = c->guard;
   switch (c->sell_shape64) {
-    case 441: launch_sell_shape<double, 4, 4, true>(c, A, epi, x, y, b, d, alpha, mg); break;
+    case 441:
+      if (sell_deep(c, A.n_slices)) launch_sell_shape<double, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg);
+      else launch_sell_shape<double, 4, 4, true>(c, A, epi, x, y, b, d, alpha, mg);
+      break;
     case 481: launch_sell_shape<double, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 841: launch_sell_shape<double, 8, 4, true>(c, A, epi, x, y, b, d, alpha, mg); break;
     default: throw Error(PM_E_INVALID, "unknown FP64 sliced SpMV shape " + std::to_string(c->sell_shape64));
@@ -1700,7 +1714,7 @@ static void launch_csr_batch_gu(pm_ctx* c, int ns, const Batch& bt, int epi, int
   c->kernel_launches++;
 }
 
-// the launch shapes DevCsr::upload picks: FP64 four lanes x four or eight
+// the launch shapes DevCsr::upload picks: FP64 two or four lanes x eight
 // loads, FP32 four x four or eight x sixteen
 template <class TV, class TX, class TA>
 static void launch_csr_batch(pm_ctx* c, int ns, const Batch& bt, int epi, int n, const DevCsr& A, const TV* v,
@@ -1708,7 +1722,8 @@ static void launch_csr_batch(pm_ctx* c, int ns, const Batch& bt, int epi, int n,
   const bool fp32 = sizeof(TV) == 4;
   const int G = fp32 ? A.lanes32 : A.lanes;
   const int U = fp32 ? A.unroll32 : A.unroll;
-  if (G == 4 && U == 4) launch_csr_batch_gu<TV, TX, TA, 4, 4>(c, ns, bt, epi, n, A, v, x, y, b, d, alpha, m);
+  if (G == 2 && U == 8) launch_csr_batch_gu<TV, TX, TA, 2, 8>(c, ns, bt, epi, n, A, v, x, y, b, d, alpha, m);
+  else if (G == 4 && U == 4) launch_csr_batch_gu<TV, TX, TA, 4, 4>(c, ns, bt, epi, n, A, v, x, y, b, d, alpha, m);
   else if (G == 4 && U == 8) launch_csr_batch_gu<TV, TX, TA, 4, 8>(c, ns, bt, epi, n, A, v, x, y, b, d, alpha, m);
   else if (G == 8 && U == 16) launch_csr_batch_gu<TV, TX, TA, 8, 16>(c, ns, bt, epi, n, A, v, x, y, b, d, alpha, m);
   else throw Error(PM_E_UNSUPPORTED, "batched CSR launch shape " + std::to_string(G) + "x" + std::to_string(U));
@@ -1721,7 +1736,10 @@ void csr_apply_batch(pm_ctx* c, const DevCsr& A, int ns, const Batch& bt, int ep
   if (A.stream && A.n_rblocks > 0) throw Error(PM_E_UNSUPPORTED, "batched launch of the streaming CSR kernel");
   if (c->sell_shape64 > 0 && A.sell64_ok && A.sell_lanes == c->sell_shape64 / 100 && A.n_slices > 0) {
     switch (c->sell_shape64) {
-      case 441: launch_sell_batch<double, 4, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask); break;
+      case 441:
+        if (sell_deep(c, (long long)A.n_slices * ns)) launch_sell_batch<double, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask);
+        else launch_sell_batch<double, 4, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask);
+        break;
       case 481: launch_sell_batch<double, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask); break;
       case 841: launch_sell_batch<double, 8, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask); break;
       default: throw Error(PM_E_INVALID, "unknown FP64 sliced SpMV shape");
@@ -1740,7 +1758,7 @@ void csr_apply32_batch(pm_ctx* c, const DevCsr& A, int ns, const Batch& bt, int 
   if (c->sell_shape > 0 && A.sell_lanes == c->sell_shape / 100 && A.n_slices > 0) {
     switch (c->sell_shape) {
       case 441: launch_sell_batch<float, 4, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
-      case 481: launch_sell_batch<float, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
+      case 481: launch_sell_batch<float, 4, 16, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
       case 841: launch_sell_batch<float, 8, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
       case 881: launch_sell_batch<float, 8, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
       default: throw Error(PM_E_UNSUPPORTED, "batched launch of sliced shape " + std::to_string(c->sell_shape));

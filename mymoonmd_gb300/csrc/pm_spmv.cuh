@@ -129,7 +129,8 @@ csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ co
 #pragma unroll
     for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c[u]);
 #pragma unroll
-    for (int u = 0; u < U; ++u) s += TA(v[u]) * TA(xv[u]);
+    for (int u = 0; u < U; ++u)
+      if (base + u * G + lane < end) s += TA(v[u]) * TA(xv[u]);
     if (base + G * U < end) load(base + G * U);
   }
 #pragma unroll
@@ -277,14 +278,17 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
   constexpr int C = 32 / L;
   pdl_trigger();
   const int s = bx * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (s >= n_slices) return;  // whole warps leave: the shuffles below stay full-warp
+  // quotients of the block's rows by one warp (below): the warps stay together
+  constexpr bool SHARE = sizeof(T) == 8 && C < 32 && EPI == EPI_JACOBI;
+  const bool have = s < n_slices;
+  if (!SHARE && !have) return;  // whole warps leave: the shuffles below stay full-warp
   const int lane = threadIdx.x & 31;
   const int p = lane % C, sub = lane / C;
   // the matrix arrays are not written by the kernels that precede a sweep:
   // their loads start before the wait for the previous kernel
-  const int row = __ldg(perm + s * C + p);  // -1: padding row of the last window
-  const int beg = __ldg(soff + s);
-  const int NT = (__ldg(soff + s + 1) - beg) >> 5;
+  const int row = have ? __ldg(perm + s * C + p) : -1;  // -1: padding row of the last window
+  const int beg = have ? __ldg(soff + s) : 0;
+  const int NT = have ? (__ldg(soff + s + 1) - beg) >> 5 : 0;
   const T* vp = svals + beg + lane;
   const int* cp = scols + beg + lane;
   T v[U];
@@ -325,7 +329,11 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
       for (int u = 0; u < U; ++u) acc = fmadd(v[u], xv[u], acc);
     }
   } else {
-    for (int t0 = 0; t0 < NT; t0 += U) {
+    // FP64: the steps past the slice's last one cost as much as the others, so
+    // the last group is apart (SpMV of 3D Q2 on 32^3 41.4 to 39.2 us)
+    constexpr bool PEEL = sizeof(T) == 8;
+    int t0 = 0;
+    for (; t0 < NT - (PEEL ? U - 1 : 0); t0 += U) {
       T vn[U], xv[U];
       int cn[U];
 #pragma unroll
@@ -343,9 +351,39 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
         c[u] = cn[u];
       }
     }
+    if (PEEL && t0 < NT) {
+      T xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (t0 + u < NT) acc = fmadd(v[u], xv[u], acc);
+    }
   }
 #pragma unroll
   for (int off = 16; off >= C; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+  if constexpr (SHARE) {
+    // An FP64 instruction holds its sub-core for about 75 clocks however few lanes
+    // take part, and a division is about ten of them: the four warps' rows (C
+    // each) are divided together. Cycle of 3D Q2, FP64: 445 to 377 us on 32^3,
+    // 132 to 123 us on 16^3
+    __shared__ T num[4 * C], den[4 * C], old[4 * C];
+    __shared__ int rows[4 * C];
+    const int w = threadIdx.x >> 5;
+    if (sub == 0) {
+      num[w * C + p] = pre_b - acc;
+      den[w * C + p] = pre_d;
+      old[w * C + p] = pre_x;
+      rows[w * C + p] = row;
+    }
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t < 4 * C && rows[t] >= 0) {
+      const T d = num[t] / den[t];
+      y[rows[t]] = old[t] + alpha * d;
+    }
+    return;
+  }
   if (row < 0 || sub != 0) return;
   if constexpr (EPI == EPI_AXPY) {
     y[row] = pre_y + alpha * acc;
