@@ -305,7 +305,7 @@ void DevCsr::make_fp32(pm_ctx* c) {
 // diagonal entry is recorded as 0 and reported by the caller
 // eight lanes per row, four column indices in flight per lane, the first match
 // of the row; the FP32 copy in the same launch. One thread per row walked its
-// indices one dependent load after another: 32 us on the 274,625 rows of 3D Q2 on 32^3, 13 us now
+// indices one dependent load after another: 32 us on the 274,625 rows of 3D Q2 on 32^3, 25 us now
 __global__ void __launch_bounds__(256)
 k_diag(int n, const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ v,
        double* __restrict__ d, float* __restrict__ d32) {

@@ -297,11 +297,26 @@ void Multigrid::coarse_solve(pm_ctx* c) {
 }
 
 // Stopping test of the iterative coarse level in one launch: |b - A x| over the
-// CSR rows (four lanes per row), one partial sum of squares per block, and the
-// last block to finish sums the partials in block order and sets the flag unless
-// the norm is above tol. As a defect, a partial-sum and a finishing kernel the
-// test took three of the five launches of an additive Vanka sweep (about 20 of
-// its 40 us on the 6^3 Stokes level).
+// CSR rows (sixteen lanes per row, so that the few hundred entries of a Stokes row
+// are a handful of rounds of loads; with four lanes the FP64 test of the 3^3 level
+// took 19 us, now 10), one partial sum of squares per block, and the last block to
+// finish sums the partials in block order and sets the flag unless the norm is
+// above tol. As a defect, a
+// partial-sum and a finishing kernel the test took three of the five launches of an
+// additive Vanka sweep (about 20 of its 40 us on the 6^3 Stokes level).
+constexpr int kStopRows = 16;  // rows per block at a time
+// sum over the block of one value per thread, fixed order; in thread 0
+__device__ __forceinline__ double stop_block_sum(double s, double* sh) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((t & 31) == 0) sh[t >> 5] = s;
+  __syncthreads();
+  double r = 0.0;
+  if (t == 0)
+    for (int w = 0; w < 8; ++w) r += sh[w];
+  return r;
+}
 template <class T>
 __global__ void __launch_bounds__(256) k_stop_if_small(int n, const int* __restrict__ rp, const int* __restrict__ ci,
                                                        const T* __restrict__ v, const T* __restrict__ x,
@@ -310,41 +325,36 @@ __global__ void __launch_bounds__(256) k_stop_if_small(int n, const int* __restr
                                                        int* __restrict__ flag) {
   pdl_enter();
   if (guarded(flag)) return;  // uniform: only the previous launch sets it
-  __shared__ double sh[256];
+  __shared__ double sh[8];
   __shared__ bool last;
-  const int t = threadIdx.x, lane = t & 3;
+  const int t = threadIdx.x, lane = t & 15;
   double s = 0.0;
-  for (int r0 = blockIdx.x * 64; r0 < n; r0 += gridDim.x * 64) {
-    const int r = r0 + (t >> 2);
+  for (int r0 = blockIdx.x * kStopRows; r0 < n; r0 += gridDim.x * kStopRows) {
+    const int r = r0 + (t >> 4);
     const int beg = r < n ? __ldg(rp + r) : 0, end = r < n ? __ldg(rp + r + 1) : 0;
     T a = T(0);
     constexpr int U = 4;
-    for (int k0 = beg; k0 < end; k0 += 4 * U) {
+    for (int k0 = beg; k0 < end; k0 += 16 * U) {
       T vv[U], xv[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int k = k0 + 4 * u + lane;
+        const int k = k0 + 16 * u + lane;
         vv[u] = k < end ? __ldg(v + k) : T(0);
         xv[u] = k < end ? x[__ldg(ci + k)] : T(0);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) a += vv[u] * xv[u];
     }
-    a += __shfl_xor_sync(0xffffffffu, a, 1);
-    a += __shfl_xor_sync(0xffffffffu, a, 2);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (r < n && lane == 0) {
       const double d = double(b[r] - a);
       s += d * d;
     }
   }
-  sh[t] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (t < w) sh[t] += sh[t + w];
-    __syncthreads();
-  }
+  s = stop_block_sum(s, sh);
   if (t == 0) {
-    part[blockIdx.x] = sh[0];
+    part[blockIdx.x] = s;
     __threadfence();
     last = atomicAdd(count, 1u) == gridDim.x - 1;
   }
@@ -352,15 +362,10 @@ __global__ void __launch_bounds__(256) k_stop_if_small(int n, const int* __restr
   if (!last) return;
   s = 0.0;
   for (int i = t; i < int(gridDim.x); i += 256) s += __ldcg(part + i);
-  sh[t] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (t < w) sh[t] += sh[t + w];
-    __syncthreads();
-  }
+  s = stop_block_sum(s, sh);
   if (t == 0) {
     *count = 0;  // for the next test
-    if (!(sqrt(sh[0]) > tol)) *flag = 1;
+    if (!(sqrt(s) > tol)) *flag = 1;
   }
 }
 
@@ -371,7 +376,7 @@ void Multigrid::coarse_iterate(pm_ctx* c) {
   // [0] the flag, [1] the finished blocks of a test
   PM_CUDA(cudaMemsetAsync(coarse_flag.p, 0, 2 * sizeof(int), c->stream));
   c->guard = coarse_flag.p;
-  const int grid = std::max(1, std::min((n + 63) / 64, kRedBlocks));
+  const int grid = std::max(1, std::min((n + kStopRows - 1) / kStopRows, kRedBlocks));
   unsigned* count = reinterpret_cast<unsigned*>(coarse_flag.p + 1);
   try {
     for (int i = 0; i < coarse_max_it; ++i) {
