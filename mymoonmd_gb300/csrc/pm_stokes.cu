@@ -12,6 +12,8 @@
 // The projected matrix is get_combined_submatrix with the pressure projection
 // (src/Matrix/BlockFEMatrix.C:1168-1345). Cell Vanka restates
 // VankaSmoother::smooth (src/Multigrid/VankaSmoother.C:110-292).
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -22,6 +24,8 @@
 #include "pm_assemble.h"
 #include "pm_stokes.h"
 #include "pm_tetra.h"
+
+namespace cg = cooperative_groups;
 
 namespace pm {
 
@@ -1945,8 +1949,13 @@ __global__ void __launch_bounds__(512) k_nodal_rhs(const int* __restrict__ guard
 // in the open: 17 us per colour.
 // One cycle on 24^3 cubes, mixed form (4 sweeps of 27 colours and the coarse
 // level): 2.2 ms with two launches per colour, 1.36 ms; on 12^3 cubes in FP64 3.13
-// and 1.80 ms. After the wait a block takes 3.6 us in FP32 (gather 1.1, residual
+// and 1.80 ms (1.50 with the split of small colours below). After the wait a block takes 3.6 us in FP32 (gather 1.1, residual
 // 1.0, solve 0.6), 11 us in FP64.
+//
+// S = 3, FP64 with few patches: a cluster of three blocks per patch, one per
+// velocity component; the residual and the local solve couple the components only
+// through the pressure's dot product, whose parts the blocks write into each other's
+// shared memory between two cluster barriers. Each block copies the patch's matrices.
 //
 // out: the additive sweep; the corrections go to the local storage, x is only
 // read.
@@ -1971,7 +1980,7 @@ __device__ __forceinline__ void load3(const double* p, double& a, double& b, dou
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <class T, int NT, int MINB>
+template <class T, int NT, int MINB, int S>
 __global__ void __launch_bounds__(NT, MINB)
 k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, int prev_cnt,
               const int* __restrict__ prev, int colour, int nu, int n, NodalPack pk, const T* __restrict__ vals,
@@ -1983,10 +1992,13 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
   __shared__ __align__(16) T rp[kNodalParts][R][4];  // partial row sums; [0] becomes the residual
   __shared__ T part[(sizeof(T) == 8 ? kNodalParts64 : 4) * 3 * kNodalMaxNodes];
   __shared__ T dot[NT];
+  __shared__ T peer[3];  // S = 3: the components' dot products
   pdl_trigger();
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int i = patches ? patches[blockIdx.x] : int(blockIdx.x);
-  const int v0 = pk.vptr[i], m = pk.vptr[i + 1] - v0, rows3 = 3 * m;
+  // S = 3: the patch's cluster has one block per velocity component
+  const int blk = int(blockIdx.x) / S, nblk = int(gridDim.x) / S, cc = S == 3 ? int(blockIdx.x) % 3 : 0;
+  const int i = patches ? patches[blk] : blk;
+  const int v0 = pk.vptr[i], m = pk.vptr[i + 1] - v0, rows3 = 3 * m, rows = S == 3 ? m : rows3;
   const int vo = pk.voff[i], io = pk.ioff[i];
   const int nv = pk.voff[i + 1] - vo, ni = pk.ioff[i + 1] - io;
   const int c0 = pk.ch0[i], nch = pk.ch0[i + 1] - c0;
@@ -2024,12 +2036,12 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
     chunk[u] = ch < nch ? pk.chunk[c0 + ch] : make_uint2(0, 0);
     crow[u] = ch < nch ? pk.row[(c0 + ch) * 8 + (lane & 7)] : 255;
   }
-  const int comp = t < rows3 ? t / m : 0, node = t < rows3 ? t - comp * m : 0;
+  const int comp = S == 3 ? cc : t < rows ? t / m : 0, node = t < rows ? (S == 3 ? t : t - comp * m) : 0;
   T tt = T(0), bb = T(0);
   int g = 0;
-  if (t < rows3) {
-    tt = tb[6 * size_t(v0) + t];
-    bb = tb[6 * size_t(v0) + rows3 + t];
+  if (t < rows) {
+    tt = tb[6 * size_t(v0) + comp * m + node];
+    bb = tb[6 * size_t(v0) + rows3 + comp * m + node];
     g = comp * nu + nodes[node];
   }
   int gn[2];
@@ -2037,13 +2049,13 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
   for (int u = 0; u < 2; ++u) gn[u] = t + u * NT < nh + nhp ? pk.halo[h0 + t + u * NT] : 0;
   // the thread's node of the previous colour's patch, if this colour leaves it
   int pn = -1, pp = -1;
-  if (int(blockIdx.x) < prev_cnt) {
-    const int ip = prev[blockIdx.x], w0 = pk.vptr[ip], mp = pk.vptr[ip + 1] - w0;
+  if (blk < prev_cnt) {
+    const int ip = prev[blk], w0 = pk.vptr[ip], mp = pk.vptr[ip + 1] - w0;
     if (t < mp) {
       pn = pk.vidx[w0 + t];
       if ((pk.mask[pn] >> colour) & 1u) pn = -1;
     }
-    if (t == 0) pp = ip;
+    if (t == 0 && cc == 0) pp = ip;
   }
   pdl_wait();
   if (guarded(guard)) {  // uniform for the whole grid
@@ -2053,24 +2065,31 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
     copy_async_wait();
     return;
   }
-  const T rhs = t < rows3 ? __ldcg(b + g) : T(0);
-  const T rhs_p = t == 0 ? __ldcg(b + 3 * nu + i) : T(0);
-  const T xp = t == 0 ? __ldcg(xs + 3 * nu + i) : T(0);
+  if constexpr (S == 3) {
+    __syncwarp();
+    cg::this_cluster().barrier_arrive();  // this block runs: its peers may write to it
+  }
+  const T rhs = t < rows ? __ldcg(b + g) : T(0);
+  const bool press = S == 3 ? t < rows : t == 0;
+  const T rhs_p = press ? __ldcg(b + 3 * nu + i) : T(0);
+  const T xp = press ? __ldcg(xs + 3 * nu + i) : T(0);
   T c1 = T(0), c2 = T(0), c3 = T(0), c4 = T(0);
   if (pn >= 0) {
-    c1 = __ldcg(xs + pn);
-    c2 = __ldcg(xs + nu + pn);
-    c3 = __ldcg(xs + 2 * nu + pn);
+    c1 = __ldcg(xs + cc * nu + pn);
+    if (S == 1) {
+      c2 = __ldcg(xs + nu + pn);
+      c3 = __ldcg(xs + 2 * nu + pn);
+    }
   }
   if (pp >= 0) c4 = __ldcg(xs + 3 * nu + pp);
   // both halo entries' loads in flight before the first store
   T hv[2][3];
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    const int e = t + u * NT, k = e < nh ? gn[u] : 3 * nu + gn[u];
+    const int e = t + u * NT, k = e < nh ? cc * nu + gn[u] : 3 * nu + gn[u];
     hv[u][0] = hv[u][1] = hv[u][2] = T(0);
     if (e < nh + nhp) hv[u][0] = __ldcg(xs + k);
-    if (e < nh) {
+    if (S == 1 && e < nh) {
       hv[u][1] = __ldcg(xs + nu + k);
       hv[u][2] = __ldcg(xs + 2 * nu + k);
     }
@@ -2080,8 +2099,10 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
     const int e = t + u * NT;
     if (e < nh) {
       hx[e] = hv[u][0];
-      hx1[e] = hv[u][1];
-      hx2[e] = hv[u][2];
+      if (S == 1) {
+        hx1[e] = hv[u][1];
+        hx2[e] = hv[u][2];
+      }
     } else if (e < nh + nhp) {
       hp[e - nh] = hv[u][0];
     }
@@ -2089,17 +2110,21 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
   for (int e = t + 2 * NT; e < nh + nhp; e += NT) {
     const int k = pk.halo[h0 + e];
     if (e < nh) {
-      hx[e] = __ldcg(xs + k);
-      hx1[e] = __ldcg(xs + nu + k);
-      hx2[e] = __ldcg(xs + 2 * nu + k);
+      hx[e] = __ldcg(xs + cc * nu + k);
+      if (S == 1) {
+        hx1[e] = __ldcg(xs + nu + k);
+        hx2[e] = __ldcg(xs + 2 * nu + k);
+      }
     } else {
       hp[e - nh] = __ldcg(xs + 3 * nu + k);
     }
   }
   if (pn >= 0) {
-    xd[pn] = c1;
-    xd[nu + pn] = c2;
-    xd[2 * nu + pn] = c3;
+    xd[cc * nu + pn] = c1;
+    if (S == 1) {
+      xd[nu + pn] = c2;
+      xd[2 * nu + pn] = c3;
+    }
   }
   if (pp >= 0) xd[3 * nu + pp] = c4;
   copy_async_wait();
@@ -2120,24 +2145,30 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
       if (u < na) {
         const T val = v[32 * u];
         r0 += val * hx[k[u]];
-        r1 += val * hx1[k[u]];
-        r2 += val * hx2[k[u]];
+        if (S == 1) {
+          r1 += val * hx1[k[u]];
+          r2 += val * hx2[k[u]];
+        }
       }
     v = sv + 32 * (na_steps + 3 * b0) + lane;
     x = sidx + 32 * (na_steps + b0) + lane;
     for (int u = 0; u < nb; ++u) {
       const T pr = hp[x[32 * u]];
-      r0 += v[96 * u] * pr;
-      r1 += v[96 * u + 32] * pr;
-      r2 += v[96 * u + 64] * pr;
+      r0 += v[96 * u + 32 * cc] * pr;
+      if (S == 1) {
+        r1 += v[96 * u + 32] * pr;
+        r2 += v[96 * u + 64] * pr;
+      }
     }
 #pragma unroll
     for (int o = 8; o <= 16; o <<= 1) {
       r0 += __shfl_xor_sync(0xffffffffu, r0, o);
-      r1 += __shfl_xor_sync(0xffffffffu, r1, o);
-      r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+      if (S == 1) {
+        r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+        r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+      }
     }
-    if (row != 255 && sub < 3) rp[pt][row][sub] = sub == 0 ? r0 : sub == 1 ? r1 : r2;
+    if (row != 255 && sub < (S == 3 ? 1 : 3)) rp[pt][row][sub] = sub == 0 ? r0 : sub == 1 ? r1 : r2;
   };
 #pragma unroll
   for (int u = 0; u < CP; ++u)
@@ -2145,11 +2176,12 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
   for (int ch = warp + CP * NW; ch < nch; ch += NW)
     residual_rows(pk.chunk[c0 + ch], pk.row[(c0 + ch) * 8 + (lane & 7)]);
   __syncthreads();
-  if (t < rows3) {
-    T s = rhs - rp[0][node][comp];
+  const int rc = S == 3 ? 0 : comp;
+  if (t < rows) {
+    T s = rhs - rp[0][node][rc];
 #pragma unroll
-    for (int k = 1; k < kNodalParts; ++k) s -= rp[k][node][comp];
-    rp[0][node][comp] = s;
+    for (int k = 1; k < kNodalParts; ++k) s -= rp[k][node][rc];
+    rp[0][node][rc] = s;
   }
   __syncthreads();
   // w = A^{-1} r: thread (q, a) sums the q-th part of row a's columns. FP64: as
@@ -2166,23 +2198,29 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
 #pragma unroll 6
     for (int k = b0; k < b1; ++k) {
       const T av = sinvm[k * m + a];
-      T x0, x1, x2;
-      load3(&rp[0][k][0], x0, x1, x2);
-      w0 += av * x0;
-      w1 += av * x1;
-      w2 += av * x2;
+      if constexpr (S == 3) {
+        w0 += av * rp[0][k][0];
+      } else {
+        T x0, x1, x2;
+        load3(&rp[0][k][0], x0, x1, x2);
+        w0 += av * x0;
+        w1 += av * x1;
+        w2 += av * x2;
+      }
     }
     T* to = part + q * rows3 + a;
     to[0] = w0;
-    to[m] = w1;
-    to[2 * m] = w2;
+    if (S == 1) {
+      to[m] = w1;
+      to[2 * m] = w2;
+    }
   }
   __syncthreads();
   T w = T(0), xo = T(0), d = T(0);
-  if (t < rows3) {
+  if (t < rows) {
     w = part[t];
     for (int q = 1; q < parts; ++q) w += part[q * rows3 + t];
-    xo = hx[comp * nh + node];
+    xo = hx[rc * nh + node];
     d = bb * (xo + w);
   }
   // one warp sums the dot product: an FP64 addition costs a warp 75 clocks of
@@ -2195,23 +2233,38 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
     for (int k = 0; k < NW; ++k) e[k] = dot[lane + 32 * k];
 #pragma unroll
     for (int k = 1; k < NW; ++k)
-      if (32 * k < rows3) e[0] += e[k];
+      if (32 * k < rows) e[0] += e[k];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) e[0] += __shfl_xor_sync(0xffffffffu, e[0], o);
     // the pressure's own residual joins it
-    if (lane == 0) dot[0] = -si * (e[0] + (cdi * xp - rhs_p));
+    if (S == 1 && lane == 0) dot[0] = -si * (e[0] + (cdi * xp - rhs_p));
+    if constexpr (S == 3) {
+      cg::cluster_group cl = cg::this_cluster();
+      __syncwarp();
+      cl.barrier_wait();  // the peers run
+      if (lane < 3) *cl.map_shared_rank(peer + cc, lane) = e[0];
+    }
   }
-  __syncthreads();
-  const T pr = dot[0];
+  T pr;
+  if constexpr (S == 3) {
+    cg::cluster_group cl = cg::this_cluster();
+    if (warp != 0) cl.barrier_wait();
+    __syncwarp();
+    cl.sync();  // nothing is written to a peer after this
+    pr = -si * ((peer[0] + peer[1] + peer[2]) + (cdi * xp - rhs_p));
+  } else {
+    __syncthreads();
+    pr = dot[0];
+  }
   const T du = damp * (w - tt * pr);
   if (out) {
     const size_t off = 3 * size_t(v0) + i;
-    if (t < rows3) out[off + t] = du;
-    if (t == 0) out[off + rows3] = damp * pr;
+    if (t < rows) out[off + comp * m + node] = du;
+    if (t == 0 && cc == 0) out[off + rows3] = damp * pr;
     return;
   }
-  if (t < rows3) xd[g] = xo + du;
-  if (t == 0) xd[3 * nu + i] = xp + damp * pr;
+  if (t < rows) xd[g] = xo + du;
+  if (t == 0 && cc == 0) xd[3 * nu + i] = xp + damp * pr;
   if (prev_cnt < 0) {
     for (int e = blockIdx.x * NT + t; e < n; e += gridDim.x * NT) {
       const int k = e < 3 * nu ? e % nu : e - 2 * nu;
@@ -2220,20 +2273,22 @@ k_nodal_patch(const int* __restrict__ guard, const int* __restrict__ patches, in
     return;
   }
   // a previous colour with more patches than this one has
-  for (int j = blockIdx.x + gridDim.x; j < prev_cnt; j += gridDim.x) {
+  for (int j = blk + nblk; j < prev_cnt; j += nblk) {
     const int ip = prev[j], w0 = pk.vptr[ip], mp = pk.vptr[ip + 1] - w0;
     for (int e = t; e < mp; e += NT) {
       const int k = pk.vidx[w0 + e];
       if ((pk.mask[k] >> colour) & 1u) continue;
-      xd[k] = __ldcg(xs + k);
-      xd[nu + k] = __ldcg(xs + nu + k);
-      xd[2 * nu + k] = __ldcg(xs + 2 * nu + k);
+      xd[cc * nu + k] = __ldcg(xs + cc * nu + k);
+      if (S == 1) {
+        xd[nu + k] = __ldcg(xs + nu + k);
+        xd[2 * nu + k] = __ldcg(xs + 2 * nu + k);
+      }
     }
-    if (t == 0) xd[3 * nu + ip] = __ldcg(xs + 3 * nu + ip);
+    if (t == 0 && cc == 0) xd[3 * nu + ip] = __ldcg(xs + 3 * nu + ip);
   }
 }
 
-template <class T, int NT, int MINB>
+template <class T, int NT, int MINB, int S>
 static void launch_nodal_patch_nt(pm_ctx* c, const DevNodalVanka& nv, int cnt, const int* patches, int prev_cnt,
                                   const int* prev, int colour, const T* vals, const T* ainv, const T* tb,
                                   const T* sinv, const T* cd, const T* b, const T* xs, T* xd, T* out, T damp) {
@@ -2243,30 +2298,49 @@ static void launch_nodal_patch_nt(pm_ctx* c, const DevNodalVanka& nv, int cnt, c
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(k_nodal_patch<T, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    attr_err = cudaFuncSetAttribute(k_nodal_patch<T, NT, MINB, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     int(kNodalPatchSmem));
   });
   PM_CUDA(attr_err);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(cnt));
+  cfg.gridDim = dim3(unsigned(cnt) * S);
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = c->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (S > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = S;
+    attr[na].val.clusterDim.y = 1;
+    attr[na++].val.clusterDim.z = 1;
+  }
+  if (c->pdl >= 1) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = c->pdl >= 1 ? 1 : 0;
-  PM_CUDA(cudaLaunchKernelEx(&cfg, k_nodal_patch<T, NT, MINB>, c->guard, patches, prev_cnt, prev, colour, nv.nu, nv.n,
+  cfg.numAttrs = unsigned(na);
+  PM_CUDA(cudaLaunchKernelEx(&cfg, k_nodal_patch<T, NT, MINB, S>, c->guard, patches, prev_cnt, prev, colour, nv.nu, nv.n,
                              pk, vals, ainv, tb, sinv, cd, b, xs, xd, out, damp));
   c->kernel_launches++;
 }
 
 // 12 warps: one chunk of the residual each for most patches
 template <class T, class... Args>
-static void launch_nodal_patch(pm_ctx* c, const DevNodalVanka& nv, Args... args) {
+static void launch_nodal_patch(pm_ctx* c, const DevNodalVanka& nv, int cnt, Args... args) {
   static_assert(4 * kNodalMaxNodes <= 384, "four threads per row, one per velocity unknown");
-  launch_nodal_patch_nt<T, 384, sizeof(T) == 4 ? 3 : 1>(c, nv, args...);
+  if constexpr (sizeof(T) == 8) {
+    // A component's block has a third of the patch's FP64 work, where it finds an SM of
+    // its own: a colour of 12 patches 18.2 to 13.7 us, 18 patches 15.8 to 12.6, 27
+    // patches 15.6 to 12.3; 64 patches (192 blocks on 152 SMs) 16.9 to 19.1, 80 patches
+    // 18.5 to 22.4. FP32 is not bound by its arithmetic
+    if (3ll * cnt <= c->num_sms) {
+      launch_nodal_patch_nt<T, 384, 2, 3>(c, nv, cnt, args...);
+      return;
+    }
+  }
+  launch_nodal_patch_nt<T, 384, sizeof(T) == 4 ? 3 : 1, 1>(c, nv, cnt, args...);
 }
 
 template <class T>

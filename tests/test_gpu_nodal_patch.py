@@ -41,3 +41,11 @@ def test_cycle_of_packed_patches(ctx, root, refine, coarse, stop, precision):
     finally:
         ctx.set_option("nodal_sliced", 8)
     assert rel(out[8], out[0]) <= (1e-12 if precision == "fp64" else 1e-5)
+
+
+@pytest.mark.parametrize("coarse", ["nodal_vanka_jacobi", "nodal_vanka"])
+@pytest.mark.parametrize("root,refine", [(3, 1), (5, 1), (7, 1), (4, 2)])
+def test_fp64_colours_around_one_block_per_sm(ctx, root, refine, coarse):
+    """colours of up to 8, 27, 64 and 64 patches: on clusters of three blocks up to a
+    third of the SMs, on one block per patch above it, both in one sweep"""
+    test_cycle_of_packed_patches(ctx, root, refine, coarse, 0.0, "fp64")
