@@ -411,12 +411,12 @@ def run_ours(args, w, rank, world, local, pg):
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "gpu_launches": mixed["launches"],
         "roofline": {"bound": "hbm",
-                     "kernel": ("sell_kernel<float,8,8,PIPE,EPI_DEFECT> on the patch rows + k_nodal_local<float>: "
+                     "kernel": ("k_nodal_patch<float,384,3,1>: "
                                 "one colour of the multiplicative nodal Vanka sweep in FP32 (local residuals of the "
-                                "colour's patches from their sliced rows, then their Schur-complement local solves "
+                                "colour's patches from their packed rows, their Schur-complement local solves "
                                 "and the update; all colours of both fine levels)"
                                 if stokes else
-                                "sell_kernel<4,8,PIPE,EPI_JACOBI>: finest-level damped Jacobi sweep in FP32 "
+                                "sell_kernel<4,16,PIPE,EPI_JACOBI>: finest-level damped Jacobi sweep in FP32 "
                                 "on the sliced-ELL copy (the largest share of a mixed request's GPU time)"),
                      "achieved": round(achieved, 1) if achieved else None, "peak": hbm_peak,
                      "unit": "GB/s", "frac": round(achieved / hbm_peak, 3) if achieved else None,
@@ -424,7 +424,7 @@ def run_ours(args, w, rank, world, local, pg):
                          round(probe_bytes / n_probe) if n_probe else None,
                      "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)",
                      "launches_probed": n_probe,
-                     "probe": (f"CUDA events around each colour's kernel pair over {min(K, 3)} requests run "
+                     "probe": (f"CUDA events around each colour's kernel over {min(K, 3)} requests run "
                                "right after the timed ones" if stokes else
                                f"CUDA events around each probed finest-level launch over {min(K, 3)} "
                                "requests run right after the timed ones")},

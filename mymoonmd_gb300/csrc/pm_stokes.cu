@@ -1103,6 +1103,8 @@ bool DevNodalVanka::build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vect
   int64_t nv32 = 0, ni32 = 0;
   pk_smem32.assign(size_t(n_colors) + 1, 0);
   pk_smem64.assign(size_t(n_colors) + 1, 0);
+  pk_elems.assign(size_t(n_colors) + 1, 0);
+  pk_index_bytes.assign(size_t(n_colors) + 1, 0);
   for (int i = 0; i < np; ++i) {
     const int m = vp[i + 1] - vp[i];
     const int* nd = vi.data() + vp[i];
@@ -1212,6 +1214,9 @@ bool DevNodalVanka::build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vect
       const int inv = (m * m + 3) & ~3, rest = 32 * (na + 3 * nb) + 3 * nh + int(hp.size()), ix = 64 * (na + nb);
       pk_smem32[k] = std::max(pk_smem32[k], 4 * (inv + rest) + ix);
       pk_smem64[k] = std::max(pk_smem64[k], 8 * (inv + rest) + ix);
+      // t, b_k, the right-hand side read and the iterate written
+      pk_elems[k] += inv + rest + 12 * m + 2;
+      pk_index_bytes[k] += ix + 4 * (nh + int(hp.size()));
     }
     if (nv32 > 0x3ffffff) return false;  // entries stay below 2^31
     voff[size_t(i) + 1] = int(nv32);
@@ -2407,11 +2412,13 @@ static bool nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T
       cudaEvent_t e0 = probe_event(c);
       PM_CUDA(cudaEventRecord(e0, c->stream));
       c->probe_events.push_back(e0);
-      // algorithmic bytes of the pair: the rows' values, column indices and
+      // algorithmic bytes of the fused kernel: what its blocks read once and write;
+      // of the pair: the rows' values, column indices and
       // gathered x, b, the local residuals written and read back, the
       // inverses (m^2), t and b vectors (6 m), 1/S, and x read and written
       const double eb = double(sizeof(T));
-      c->probe_bytes.push_back(double(nv.color_entries[k]) * (2 * eb + 4) + double(nv.color_rows[k]) * 5 * eb +
+      if (fused) c->probe_bytes.push_back(double(nv.pk_elems[k]) * eb + double(nv.pk_index_bytes[k]));
+      else c->probe_bytes.push_back(double(nv.color_entries[k]) * (2 * eb + 4) + double(nv.color_rows[k]) * 5 * eb +
                                double(nv.color_msq[k]) * eb + double(nv.color_nodes[k]) * 6 * eb + double(cnt) * eb);
     }
     if (fused) {

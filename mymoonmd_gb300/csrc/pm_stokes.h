@@ -181,6 +181,7 @@ struct DevNodalVanka {
   // per colour and (last entry) over all patches: shared memory of a block, for
   // FP32 and FP64 values
   std::vector<int> pk_smem32, pk_smem64;
+  std::vector<int64_t> pk_elems, pk_index_bytes;  // per colour: values, index bytes moved
   int64_t pk_entries = 0;               // packed values
   DBuf<int> pk_voff, pk_ioff;           // per patch: values and indices, in units of 32 (np + 1)
   DBuf<uint2> pk_chunk;                 // NodalChunk of every warp's share
