@@ -1115,6 +1115,9 @@ __device__ __forceinline__ void gj_warp_best(unsigned long long& key, int& pos, 
 // (panel rows: 0) + (D | W) * (pivot rows of src); after the last panel the
 // columns go where the row swaps belong in the inverse (out[i][rowsrc[j]]).
 //
+// Both are launched early and read what the launch before them writes (the matrix,
+// D, prm, rowsrc): plain pointers, no trigger before the wait.
+//
 // The chain of columns bounds it. A thread-block cluster with one cluster
 // barrier and one remote row per column took 4 to 8 us per column.
 // Update of a two-level solver (the rest of it takes about 85 us), cluster or
@@ -1124,9 +1127,8 @@ __device__ __forceinline__ void gj_warp_best(unsigned long long& key, int& pos, 
 constexpr int kGjMaxRows = 4096;
 
 template <class T, int NB, int RPT>
-__global__ void __launch_bounds__(1024) k_gj_panel(int n, int k0, int nb, const T* __restrict__ M, T* __restrict__ D,
-                                                   T* __restrict__ steps, int* __restrict__ prm, int* __restrict__ rowsrc,
-                                                   int* __restrict__ flag) {
+__global__ void __launch_bounds__(1024) k_gj_panel(int n, int k0, int nb, const T* M, T* D, T* steps, int* prm,
+                                                   int* rowsrc, int* flag) {
   constexpr bool WIDE = sizeof(T) == 8;
   // by the parity of the step: the warps' candidates (key, position, row) and
   // the row at the step's position
@@ -1135,7 +1137,8 @@ __global__ void __launch_bounds__(1024) k_gj_panel(int n, int k0, int nb, const 
   __shared__ int wpos[2][32];
   extern __shared__ int sp[];  // row at each position
   const int t = threadIdx.x, bd = blockDim.x, lane = t & 31, warp = t >> 5, nw = bd >> 5;
-  pdl_enter();
+  pdl_wait();
+  pdl_trigger();
   T row[RPT][NB];
 #pragma unroll
   for (int s = 0; s < RPT; ++s) {
@@ -1247,16 +1250,15 @@ __global__ void __launch_bounds__(1024) k_gj_panel(int n, int k0, int nb, const 
 
 // TR x 32 tile per block of 32 x 8 threads; cols: the last panel's column map
 template <class T, int NB, int TR>
-__global__ void __launch_bounds__(256) k_gj_apply(int n, int k0, int nb, const T* __restrict__ src,
-                                                  const T* __restrict__ D, const T* __restrict__ steps,
-                                                  const int* __restrict__ prm, const int* __restrict__ cols,
-                                                  T* __restrict__ dst) {
+__global__ void __launch_bounds__(256) k_gj_apply(int n, int k0, int nb, const T* src, const T* D, const T* steps,
+                                                  const int* prm, const int* cols, T* dst) {
   constexpr int QR = TR / 8;
   static_assert(256 % NB == 0 && NB <= 32 && (TR * NB) % 32 == 0, "one thread per panel entry, rows within a warp");
   __shared__ T w[TR][NB + 1], piv[NB][32], st[NB][NB];
   const int tx = threadIdx.x, ty = threadIdx.y, t = ty * 32 + tx;
   const int i0 = blockIdx.y * TR, j = blockIdx.x * 32 + tx;
-  pdl_enter();
+  pdl_wait();
+  pdl_trigger();
   for (int e = t; e < NB * NB; e += 256) st[e / NB][e % NB] = e / NB < nb ? steps[e] : T(0);
   for (int l = ty; l < NB; l += 8) piv[l][tx] = (l < nb && j < n) ? src[(size_t)prm[k0 + l] * n + j] : T(0);
   T acc[QR];
@@ -1636,8 +1638,8 @@ namespace pm {
 template <class TV, class TX, class TA, int G, int U, int EPI>
 __global__ void __launch_bounds__(256)
 csr_batch_kernel(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ cols,
-                 const TV* __restrict__ vals, const TX* __restrict__ x, TX* __restrict__ y,
-                 const TX* __restrict__ b, const TX* __restrict__ diag, TA alpha, BlockMask mask, Batch bt) {
+                 const TV* __restrict__ vals, const TX* x, TX* y, const TX* b, const TX* __restrict__ diag,
+                 TA alpha, BlockMask mask, Batch bt) {
   const int s = blockIdx.x;
   if (!bt.on[s]) return;
   const TV* v = bt.vals ? static_cast<const TV*>(bt.vals[2 * s + 1]) : vals;
@@ -1650,9 +1652,8 @@ csr_batch_kernel(int n_rows, const int* __restrict__ row_ptr, const int* __restr
 template <class T, int L, int U, bool PIPE, int EPI>
 __global__ void __launch_bounds__(128)
 sell_batch_kernel(int n_slices, const int* __restrict__ perm, const int* __restrict__ soff,
-                  const int* __restrict__ scols, const T* __restrict__ svals, const T* __restrict__ x,
-                  T* __restrict__ y, const T* __restrict__ b, const T* __restrict__ diag, T alpha, BlockMask mask,
-                  Batch bt) {
+                  const int* __restrict__ scols, const T* __restrict__ svals, const T* x, T* y, const T* b,
+                  const T* __restrict__ diag, T alpha, BlockMask mask, Batch bt) {
   const int s = blockIdx.x;
   if (!bt.on[s]) return;
   const T* v = bt.vals ? static_cast<const T*>(bt.vals[2 * s]) : svals;

@@ -56,6 +56,17 @@ __device__ __forceinline__ T ld_stream(const T* p) { return __ldcs(p); }
 // stream (if launched with programmatic stream serialization) start once all
 // blocks of this one have started; pdl_wait blocks until the previous kernel
 // has completed and its writes are visible (a no-op without the attribute).
+//
+// A kernel launched that way is resident while the one before it still writes,
+// so what earlier kernels of the stream write is not constant over its lifetime:
+// it reads such data after pdl_wait, through plain pointers (a __restrict__ const
+// pointer or __ldg gives ld.global.nc, which is for constant data only; the matrix
+// arrays, written before the first early launch, keep it). It triggers after the
+// wait, so that its successor starts when its predecessor is done: with the
+// trigger first, a third kernel could run beside the first one, whose reads of the
+// buffer that the second writes stay in an SM's L1. The later trigger costs
+// nothing: cycle of 2D Q1 on 32^2 60.7 us with the trigger first and 59.8 after the
+// wait, of 3D Q2 on 16^3 105.3 and 102.3.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the start of a kernel launched by launch_k that reads nothing before the
@@ -81,10 +92,8 @@ __device__ __forceinline__ double fmadd<double>(double a, double b, double c) { 
 template <class TV, class TX, class TA, int G, int U, int EPI>
 __device__ __forceinline__ void
 csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ cols,
-         const TV* __restrict__ vals, const TX* __restrict__ x, TX* __restrict__ y,
-         const TX* __restrict__ b, const TX* __restrict__ diag, const TX* __restrict__ xold,
-         TA alpha, const BlockMask& mask, int bx, int gx) {
-  pdl_trigger();
+         const TV* __restrict__ vals, const TX* x, TX* y, const TX* b, const TX* __restrict__ diag,
+         const TX* xold, TA alpha, const BlockMask& mask, int bx, int gx) {
   const int lane = threadIdx.x & (G - 1);
   const int row = (bx * blockDim.x + threadIdx.x) / G;
   const bool valid = row < n_rows;  // whole groups share a row: no early exit before the shuffles
@@ -107,6 +116,7 @@ csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ co
   };
   if (beg < end) load(beg);
   pdl_wait();
+  pdl_trigger();
   if (guarded(mask.guard)) {  // uniform for the whole grid
     // a skipped Jacobi sweep leaves the iterate as it is (the caller swaps
     // the two iterate buffers after every sweep)
@@ -119,15 +129,15 @@ csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ co
   TX pre_b = TX(0), pre_d = TX(1), pre_x = TX(0), pre_y = TX(0);
   if (valid && lane == 0) {
     if constexpr (EPI == EPI_AXPY || EPI == EPI_PROLONG) pre_y = y[row];
-    if constexpr (EPI == EPI_DEFECT || EPI == EPI_JACOBI) pre_b = __ldg(b + row);
+    if constexpr (EPI == EPI_DEFECT || EPI == EPI_JACOBI) pre_b = b[row];
     if constexpr (EPI == EPI_JACOBI || EPI == EPI_RESTRICT_ZERO) pre_d = __ldg(diag + row);
-    if constexpr (EPI == EPI_JACOBI) pre_x = __ldg(xold + row);
+    if constexpr (EPI == EPI_JACOBI) pre_x = xold[row];
   }
   TA s = TA(0);
   for (int base = beg; base < end; base += G * U) {
     TX xv[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c[u]);
+    for (int u = 0; u < U; ++u) xv[u] = x[c[u]];
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (base + u * G + lane < end) s += TA(v[u]) * TA(xv[u]);
@@ -160,9 +170,8 @@ csr_body(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ co
 template <class TV, class TX, class TA, int G, int U, int EPI>
 __global__ void __launch_bounds__(256)
 csr_kernel(int n_rows, const int* __restrict__ row_ptr, const int* __restrict__ cols,
-           const TV* __restrict__ vals, const TX* __restrict__ x, TX* __restrict__ y,
-           const TX* __restrict__ b, const TX* __restrict__ diag, const TX* __restrict__ xold,
-           TA alpha, BlockMask mask) {
+           const TV* __restrict__ vals, const TX* x, TX* y, const TX* b, const TX* __restrict__ diag,
+           const TX* xold, TA alpha, BlockMask mask) {
   csr_body<TV, TX, TA, G, U, EPI>(n_rows, row_ptr, cols, vals, x, y, b, diag, xold, alpha, mask, blockIdx.x,
                                   gridDim.x);
 }
@@ -272,11 +281,9 @@ constexpr int kSellWindow = 1024;
 template <class T, int L, int U, bool PIPE, int EPI>
 __device__ __forceinline__ void
 sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ soff,
-          const int* __restrict__ scols, const T* __restrict__ svals, const T* __restrict__ x,
-          T* __restrict__ y, const T* __restrict__ b, const T* __restrict__ diag, T alpha,
-          const BlockMask& mask, int bx) {
+          const int* __restrict__ scols, const T* __restrict__ svals, const T* x, T* y, const T* b,
+          const T* __restrict__ diag, T alpha, const BlockMask& mask, int bx) {
   constexpr int C = 32 / L;
-  pdl_trigger();
   const int s = bx * (blockDim.x >> 5) + (threadIdx.x >> 5);
   // quotients of the block's rows by one warp (below): the warps stay together
   constexpr bool SHARE = sizeof(T) == 8 && C < 32 && EPI == EPI_JACOBI;
@@ -302,6 +309,7 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
     }
   }
   pdl_wait();  // x, b, y and the guard flag come from earlier kernels
+  pdl_trigger();
   if (guarded(mask.guard)) {  // uniform for the whole grid
     if (EPI == EPI_JACOBI && row >= 0 && sub == 0) y[row] = x[row];
     return;
@@ -309,9 +317,9 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
   T pre_b = T(0), pre_d = T(1), pre_x = T(0), pre_y = T(0);
   if (row >= 0 && sub == 0) {
     if constexpr (EPI == EPI_AXPY || EPI == EPI_PROLONG) pre_y = y[row];
-    if constexpr (EPI == EPI_DEFECT || EPI == EPI_JACOBI) pre_b = __ldg(b + row);
+    if constexpr (EPI == EPI_DEFECT || EPI == EPI_JACOBI) pre_b = b[row];
     if constexpr (EPI == EPI_JACOBI || EPI == EPI_RESTRICT_ZERO) pre_d = __ldg(diag + row);
-    if constexpr (EPI == EPI_JACOBI) pre_x = __ldg(x + row);
+    if constexpr (EPI == EPI_JACOBI) pre_x = x[row];
   }
   T acc = T(0);
   if constexpr (!PIPE) {
@@ -324,7 +332,7 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
         c[u] = in ? ld_stream(cp + (t0 + u) * 32) : 0;
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c[u]);
+      for (int u = 0; u < U; ++u) xv[u] = x[c[u]];
 #pragma unroll
       for (int u = 0; u < U; ++u) acc = fmadd(v[u], xv[u], acc);
     }
@@ -343,7 +351,7 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
         cn[u] = in ? ld_stream(cp + (t0 + U + u) * 32) : 0;
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c[u]);
+      for (int u = 0; u < U; ++u) xv[u] = x[c[u]];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         acc = fmadd(v[u], xv[u], acc);
@@ -354,7 +362,7 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
     if (PEEL && t0 < NT) {
       T xv[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = __ldg(x + c[u]);
+      for (int u = 0; u < U; ++u) xv[u] = x[c[u]];
 #pragma unroll
       for (int u = 0; u < U; ++u)
         if (t0 + u < NT) acc = fmadd(v[u], xv[u], acc);
@@ -408,9 +416,8 @@ sell_body(int n_slices, const int* __restrict__ perm, const int* __restrict__ so
 template <class T, int L, int U, bool PIPE, int EPI>
 __global__ void __launch_bounds__(128)
 sell_kernel(int n_slices, const int* __restrict__ perm, const int* __restrict__ soff,
-            const int* __restrict__ scols, const T* __restrict__ svals, const T* __restrict__ x,
-            T* __restrict__ y, const T* __restrict__ b, const T* __restrict__ diag, T alpha,
-            BlockMask mask) {
+            const int* __restrict__ scols, const T* __restrict__ svals, const T* x, T* y, const T* b,
+            const T* __restrict__ diag, T alpha, BlockMask mask) {
   sell_body<T, L, U, PIPE, EPI>(n_slices, perm, soff, scols, svals, x, y, b, diag, alpha, mask, blockIdx.x);
 }
 

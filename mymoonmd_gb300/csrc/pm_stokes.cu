@@ -1941,8 +1941,10 @@ __global__ void __launch_bounds__(512) k_nodal_rhs(const int* __restrict__ guard
 // from xs to xd. xd already holds xs as of one colour before, so besides its own
 // nodes a block moves the nodes of one patch of the previous colour that this
 // colour does not update (the first colour: its share of all of them).
-// The iterate is read from L2 (ld.cg): up to three colours' kernels are in flight
-// and the first of them may have left lines of xd's buffer in an SM's L1.
+// The kernel triggers its successor before it waits, so up to three colours' kernels
+// are in flight, and the first of them reads the buffer that the second one writes
+// and the third reads: the iterate is read from L2 (ld.cg), past the lines that an
+// SM's L1 may hold.
 //
 // The inverse and the packed rows are copied to shared memory (cp.async) before
 // the wait for the previous colour's kernel (programmatic dependent launch), so
