@@ -262,6 +262,7 @@ void DevCsr::values_changed(pm_ctx* c) {
     PM_CHECK_LAUNCH();
     c->kernel_launches++;
     sell64_ok = true;
+    sell_fresh = true;
   }
 }
 
@@ -284,6 +285,7 @@ void DevCsr::make_fp32(pm_ctx* c) {
                                                                        sell_vals.p);
     PM_CHECK_LAUNCH();
     c->kernel_launches++;
+    sell_fresh = true;
   }
   vals32.ensure(size_t(nnz4()));
   if (nnz4() > nnz)
@@ -431,7 +433,10 @@ static void launch_sell_epi(pm_ctx* c, const DevCsr& A, const T* x, T* y, const 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = c->pdl >= 1 ? 1 : 0;
+  // plainly after a fill of the sliced values, so that this launch and the early ones
+  // after it find them complete (a cycle's first kernel is launched plainly)
+  cfg.numAttrs = c->pdl >= 1 && (c->in_cycle || !A.sell_fresh) ? 1 : 0;
+  A.sell_fresh = false;
   PM_CUDA(cudaLaunchKernelEx(&cfg, sell_kernel<T, L, U, P, EPI>, A.n_slices, (const int*)A.sell_perm.p,
                              (const int*)A.sell_off.p, (const int*)A.sell_cols.p, sell_values<T>(A), x, y, b, d,
                              alpha, m));

@@ -63,6 +63,9 @@ struct DevCsr {
   // current values (every writer of vals calls values_changed)
   DBuf<double> sell_vals64;
   bool sell64_ok = false;
+  // the sliced values were filled and no launch has followed the fill yet: a sweep
+  // that is launched early loads them before its wait, when the fill may still write
+  mutable bool sell_fresh = false;
   BlockMask mask{};
   DBuf<int> row_ptr, cols;
   DBuf<double> vals;

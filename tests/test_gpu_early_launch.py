@@ -95,3 +95,34 @@ def test_direct_solves_have_the_bits_of_plain_launches(ctx, n):
     plain, early = both(ctx, run)
     A.close()
     assert (plain == plain[0]).all() and np.array_equal(plain, early)
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+def test_product_right_after_new_values(ctx, fp32):
+    """the first product after the sliced values were filled, launch after launch"""
+    disc = m.Discretization(m.GEO_CUBE_HEXA, 1, 4, 1, m.KIND_CD, 2, ctx=ctx)
+    db = cd_db("fp64", 1)
+    db["preconditioner"] = "no_preconditioner"
+    prob = m.ConvectionDiffusion(ctx, disc, m.cd_coeffs(0.1, (1.0, 0.5, 0.25), 0.0, True), db, quad_points=3)
+    prob.assemble()
+    A = prob.matrix(-1)
+    A.make_sliced64()
+    v, n = A.values(), A.n_rows
+    dtype = np.float32 if fp32 else np.float64
+    x = m.DeviceVector.from_numpy(ctx, np.random.default_rng(1).standard_normal(n).astype(dtype))
+    y = m.DeviceVector(ctx, n, dtype)
+
+    def product(scale):
+        A.set_values(scale * v)  # a power of two: the products scale exactly
+        if fp32:
+            A.make_fp32()
+            A.apply_f32(x, y)
+        else:
+            A.apply(x, y)
+        return y.numpy()
+
+    one = product(1.0)
+    for k in range(1, 40):
+        assert np.array_equal(product(2.0 ** (k % 7)), one * dtype(2.0 ** (k % 7)))
+    prob.close()
+    disc.close()
