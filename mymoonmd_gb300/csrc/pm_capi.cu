@@ -311,7 +311,10 @@ int pm_matrix_get_structure(const pm_matrix* A, int* rp, int* ci) {
   if (!A) return PM_E_INVALID;
   PM_TRY
   if (rp) A->csr.row_ptr.download(rp, A->ctx->stream);
-  if (ci) A->csr.cols.download(ci, A->ctx->stream);
+  // the device array is padded to a multiple of four entries
+  if (ci && A->csr.nnz)
+    PM_CUDA(cudaMemcpyAsync(ci, A->csr.cols.p, size_t(A->csr.nnz) * sizeof(int), cudaMemcpyDeviceToHost,
+                            A->ctx->stream));
   PM_CUDA(cudaStreamSynchronize(A->ctx->stream));
   return PM_OK;
   PM_CATCH(A->ctx)
