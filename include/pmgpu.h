@@ -73,7 +73,7 @@ int pm_version(void);
  *   sweeps (counted as one launch, with the pair's algorithmic bytes);
  *   "nodal_sliced" 0|4|8 - nodal Vanka sweeps by one kernel per colour over
  *   packed patches (8, default; packed when a problem sets up its smoothers, up
- *   to 32 colours), or with the local residuals of a colour by one sliced-ELL
+ *   to 32 colours; a matrix whose velocity blocks differ is swept as with 0), or with the local residuals of a colour by one sliced-ELL
  *   launch over a copy of its patches' rows (4, 1 = 4; also 8 where the patches
  *   do not fit the kernel) or by one block per patch over the CSR rows (0); the
  *   copies' values are refreshed with the Vanka factors;

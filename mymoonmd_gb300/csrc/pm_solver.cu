@@ -1165,6 +1165,8 @@ size_t pm_solver::layout_signature() const {
     mix(lv.coarse_rhs64.p); mix(lv.coarse_sol64.p);
     mix(lv.sor.rows.p);
     h ^= lv.sor.ptr.size();
+    // the nodal sweep's kernels depend on the matrix (equal velocity blocks)
+    if (lv.nodal) h = h * 1099511628211ull ^ size_t(lv.nodal->pk_same ? 2 : 1);
   }
   // the SOR preconditioner's colours (a new structure gives new launches)
   mix(sor.rows.p);

@@ -1088,7 +1088,8 @@ constexpr int kNodalSteps = 9, kNodalParts = 3;
 
 // The patches packed for k_nodal_patch. False if they do not fit it: more than
 // 32 colours (the mask's bits), longer rows than kNodalParts chunks, velocity
-// components that couple or differ.
+// components that couple or whose rows have other columns. (Velocity blocks of other
+// values: factor() looks at them, and the sweeps then go over the CSR rows.)
 bool DevNodalVanka::build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vector<int>& vp,
                                const std::vector<int>& vi, const std::vector<int>& color, int n_colors) {
   if (n_colors > 32 || max_nodes > kNodalMaxNodes) return false;
@@ -1123,8 +1124,15 @@ bool DevNodalVanka::build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vect
     lenp.assign(m, 0);
     for (int a = 0; a < m; ++a) {
       const int r0 = S.row_ptr[nd[a]], r1 = S.row_ptr[nd[a] + 1];
-      for (int k = 1; k < 3; ++k)
-        if (S.row_ptr[k * nu + nd[a] + 1] - S.row_ptr[k * nu + nd[a]] != r1 - r0) return false;
+      // the other components' rows: the same columns, moved to their own component
+      for (int k = 1; k < 3; ++k) {
+        const int q0 = S.row_ptr[k * nu + nd[a]];
+        if (S.row_ptr[k * nu + nd[a] + 1] - q0 != r1 - r0) return false;
+        for (int e = 0; e < r1 - r0; ++e) {
+          const int col = S.cols[r0 + e];
+          if (S.cols[q0 + e] != (col < nu ? col + k * nu : col)) return false;
+        }
+      }
       for (int k = r0; k < r1; ++k) {
         const int col = S.cols[k];
         if (col < nu) {
@@ -1386,7 +1394,7 @@ void DevNodalVanka::setup(pm_ctx* c, const DiscLevel& L) {
     color_nodes[k] += m;
     color_msq[k] += int64_t(m) * m;
   }
-  flag.ensure(1);
+  flag.ensure(2);
 }
 
 }  // namespace pm
@@ -1676,9 +1684,33 @@ static void launch_nodal_factor(pm_ctx* c, DevNodalVanka& nv, const int* rp, con
   else launch_nodal_factor_tr<T, 6>(c, nv, rp, ci, v, ainv, tb, sinv, cd, packed);
 }
 
+// flag = 1 unless the velocity blocks of the components hold the same values: a
+// program may write its own into the pattern (pm_matrix_set_values). Eight lanes per
+// row of the first component; bits compared as integers (FP64 compares run on the
+// FP64 pipe).
+__global__ void __launch_bounds__(256) k_same_blocks(int nu, const int* __restrict__ rp, const int* __restrict__ ci,
+                                                     const double* __restrict__ v, int* __restrict__ flag) {
+  const int lane = threadIdx.x & 7, r = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  if (r >= nu) return;
+  const int r0 = rp[r], len = rp[r + 1] - r0, r1 = rp[nu + r], r2 = rp[2 * nu + r];
+  const double *v1 = v + r1, *v2 = v + r2;
+  bool same = rp[nu + r + 1] - r1 == len && rp[2 * nu + r + 1] - r2 == len;
+  for (int k = lane; k < len && same; k += 8) {
+    if (ci[r0 + k] >= nu) continue;
+    const long long a = __double_as_longlong(v[r0 + k]);
+    same = same && a == __double_as_longlong(v1[k]) && a == __double_as_longlong(v2[k]);
+  }
+  if (!same) *flag = 1;
+}
+
 void DevNodalVanka::factor(pm_ctx* c, const DevCsr& V, bool fp32) {
-  PM_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), c->stream));
+  // [0] a singular patch, [1] the velocity blocks differ
+  PM_CUDA(cudaMemsetAsync(flag.p, 0, 2 * sizeof(int), c->stream));
   if (pk_ok) {
+    k_same_blocks<<<unsigned((8ll * nu + 255) / 256), 256, 0, c->stream>>>(nu, V.row_ptr.p, V.cols.p, V.vals.p,
+                                                                           flag.p + 1);
+    PM_CHECK_LAUNCH();
+    c->kernel_launches++;
     // the packed rows take the projected matrix's values (FP32: rounded FP64)
     const int g = int(std::max<int64_t>(1, std::min<int64_t>((pk_entries + 255) / 256, int64_t(c->num_sms) * 8)));
     if (fp32) {
@@ -1725,10 +1757,11 @@ void DevNodalVanka::factor(pm_ctx* c, const DevCsr& V, bool fp32) {
     PM_CHECK_LAUNCH();
     c->kernel_launches++;
   }
-  int h = 0;
-  PM_CUDA(cudaMemcpyAsync(&h, flag.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  int h[2] = {0, 0};
+  PM_CUDA(cudaMemcpyAsync(h, flag.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   PM_CUDA(cudaStreamSynchronize(c->stream));
-  if (h) throw Error(PM_E_BREAKDOWN, "singular local nodal Vanka system");
+  pk_same = pk_ok && !h[1];
+  if (h[0]) throw Error(PM_E_BREAKDOWN, "singular local nodal Vanka system");
 }
 
 }  // namespace pm
@@ -2353,7 +2386,7 @@ static void launch_nodal_patch(pm_ctx* c, const DevNodalVanka& nv, int cnt, Args
 template <class T>
 static void nodal_jacobi(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T* vals, const T* ainv, const T* tb,
                          const T* sinv, const T* cd, T* sol, const T* b, T* x, T* r, T damp) {
-  if (nv.pk_ok && vals && c->nodal_sliced == 8) {
+  if (nv.pk_same && vals && c->nodal_sliced == 8) {
     launch_nodal_patch<T>(c, nv, nv.np, nullptr, 0, nullptr, 0, vals, ainv, tb, sinv, cd, b, (const T*)x, nullptr,
                           sol, damp);
   } else {
@@ -2392,7 +2425,7 @@ static bool nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T
     rsv = nv.rs_vals.p;
     bl = nv.bloc.p;
   }
-  const bool fused = nv.pk_ok && packed && other && c->nodal_sliced == 8;
+  const bool fused = nv.pk_same && packed && other && c->nodal_sliced == 8;
   const bool sliced = nv.rs_ok && rsv && bl && c->nodal_sliced != 0;
   BlockMask mg{};
   mg.guard = c->guard;

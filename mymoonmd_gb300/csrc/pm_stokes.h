@@ -176,8 +176,10 @@ struct DevNodalVanka {
   DBuf<int> rs_perm, rs_off, rs_cols, rs_src, bslot;
   DBuf<float> rs_vals32, bloc32;
   DBuf<double> rs_vals, bloc;
-  // the patches packed for k_nodal_patch (see there), when they fit it
-  bool pk_ok = false;
+  // the patches packed for k_nodal_patch (see there), when they fit it; pk_same: the
+  // three velocity blocks of the current matrix are equal, so that the packed values
+  // of the first one stand for all (k_same_blocks, with every factor())
+  bool pk_ok = false, pk_same = false;
   // per colour and (last entry) over all patches: shared memory of a block, for
   // FP32 and FP64 values
   std::vector<int> pk_smem32, pk_smem64;
