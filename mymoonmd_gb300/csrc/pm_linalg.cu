@@ -2,7 +2,6 @@
 // the dense coarse-grid inverse.
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include <cooperative_groups.h>
 

@@ -17,7 +17,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -1085,6 +1084,7 @@ static NodalPack nodal_pack(const DevNodalVanka& nv) {
 // A steps per chunk (a long row's steps go to several warps) and partial sums
 // per row
 constexpr int kNodalSteps = 9, kNodalParts = 3;
+static void allow_nodal_patch_smem();
 
 // The patches packed for k_nodal_patch. False if they do not fit it: more than
 // 32 colours (the mask's bits), longer rows than kNodalParts chunks, velocity
@@ -1379,7 +1379,10 @@ void DevNodalVanka::setup(pm_ctx* c, const DiscLevel& L) {
   color_patches.upload(cp, c->stream);
   pk_ok = c->nodal_sliced == 8 && build_pack(c, S, vp, vi, color, n_colors) &&
           size_t(std::max(pk_smem32.back(), pk_smem64.back())) <= kNodalPatchSmem;
-  if (!pk_ok) build_row_slices(c, S, L.pressure_row0, vp, vi, cp);
+  // here, for every set-up: the limit belongs to the context's device, and a process
+  // may hold contexts on several
+  if (pk_ok) allow_nodal_patch_smem();
+  else build_row_slices(c, S, L.pressure_row0, vp, vi, cp);
   color_entries.assign(n_colors, 0);
   color_rows.assign(n_colors, 0);
   color_nodes.assign(n_colors, 0);
@@ -2335,13 +2338,6 @@ static void launch_nodal_patch_nt(pm_ctx* c, const DevNodalVanka& nv, int cnt, c
   const NodalPack pk = nodal_pack(nv);
   const std::vector<int>& need = sizeof(T) == 4 ? nv.pk_smem32 : nv.pk_smem64;
   const size_t smem = size_t(patches ? need[size_t(colour)] : need.back());
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(k_nodal_patch<T, NT, MINB, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(kNodalPatchSmem));
-  });
-  PM_CUDA(attr_err);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(cnt) * S);
   cfg.blockDim = dim3(NT);
@@ -2366,21 +2362,32 @@ static void launch_nodal_patch_nt(pm_ctx* c, const DevNodalVanka& nv, int cnt, c
   c->kernel_launches++;
 }
 
-// 12 warps: one chunk of the residual each for most patches
+constexpr int kPatchThreads = 384;  // 12 warps: one chunk of the residual each for most patches
+
+// the kernels' shared memory limit on the current device
+static void allow_nodal_patch_smem() {
+  auto allow = [](const void* kern) {
+    PM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kNodalPatchSmem)));
+  };
+  allow((const void*)k_nodal_patch<float, kPatchThreads, 3, 1>);
+  allow((const void*)k_nodal_patch<double, kPatchThreads, 1, 1>);
+  allow((const void*)k_nodal_patch<double, kPatchThreads, 2, 3>);
+}
+
 template <class T, class... Args>
 static void launch_nodal_patch(pm_ctx* c, const DevNodalVanka& nv, int cnt, Args... args) {
-  static_assert(4 * kNodalMaxNodes <= 384, "four threads per row, one per velocity unknown");
+  static_assert(4 * kNodalMaxNodes <= kPatchThreads, "four threads per row, one per velocity unknown");
   if constexpr (sizeof(T) == 8) {
     // A component's block has a third of the patch's FP64 work, where it finds an SM of
     // its own: a colour of 12 patches 18.2 to 13.7 us, 18 patches 15.8 to 12.6, 27
     // patches 15.6 to 12.3; 64 patches (192 blocks on 152 SMs) 16.9 to 19.1, 80 patches
     // 18.5 to 22.4. FP32 is not bound by its arithmetic
     if (3ll * cnt <= c->num_sms) {
-      launch_nodal_patch_nt<T, 384, 2, 3>(c, nv, cnt, args...);
+      launch_nodal_patch_nt<T, kPatchThreads, 2, 3>(c, nv, cnt, args...);
       return;
     }
   }
-  launch_nodal_patch_nt<T, 384, sizeof(T) == 4 ? 3 : 1, 1>(c, nv, cnt, args...);
+  launch_nodal_patch_nt<T, kPatchThreads, sizeof(T) == 4 ? 3 : 1, 1>(c, nv, cnt, args...);
 }
 
 template <class T>
