@@ -1303,8 +1303,16 @@ __global__ void __launch_bounds__(256) k_gj_apply(int n, int k0, int nb, const T
   }
 }
 
+// the matrix of gj_panels goes from buffer to buffer, panel by panel, so that the last
+// panel writes `out`: where it starts (a third buffer of n x n held 134 MB more at
+// 4,096 rows, for the solver's life)
+template <class T>
+static T* gj_start(int n, int width, T* work, T* out) { return ((n + width - 1) / width) % 2 ? work : out; }
+
+// the matrix in gj_start(n, NB, work, out); d: the panel, behind the n x n of work
 template <class T, int NB, int RPT, int TR>
-static void gj_panels(pm_ctx* c, int n, T* a, T* b, T* d, int* prm, int* rowsrc, int* flag, T* out) {
+static void gj_panels(pm_ctx* c, int n, T* work, int* prm, int* rowsrc, int* flag, T* out) {
+  T *a = gj_start(n, NB, work, out), *b = a == work ? out : work, *d = work + size_t(n) * n;
   const dim3 grid((n + 31) / 32, (n + TR - 1) / TR), block(32, 8);
   const size_t smem = size_t(n) * sizeof(int);
   for (int k0 = 0; k0 < n; k0 += NB) {
@@ -1320,7 +1328,7 @@ static void gj_panels(pm_ctx* c, int n, T* a, T* b, T* d, int* prm, int* rowsrc,
       launch_pdl(c, k_gj_panel<T, NB, RPT>, dim3(1), dim3(1024), smem, n, k0, nb, a, d, d + NB * NB, prm, rowsrc,
                  flag);
     launch_pdl(c, k_gj_apply<T, NB, TR>, grid, block, 0, n, k0, nb, a, d, d + NB * NB, prm,
-               last ? rowsrc : nullptr, last ? out : b);
+               last ? rowsrc : nullptr, b);
     std::swap(a, b);
   }
 }
@@ -1328,12 +1336,12 @@ static void gj_panels(pm_ctx* c, int n, T* a, T* b, T* d, int* prm, int* rowsrc,
 // Panel widths, by the same update: FP64 343 rows 910 / 822 / 962 us with 4 / 8 /
 // 16 columns (a step's FP64 work grows with the width, the launches fall with
 // it); FP32 469 / 416 / 459 us with 8 / 16 / 32 (with W formed from D).
-static void gj_inverse(pm_ctx* c, int n, float* a, float* b, float* d, int* prm, int* rowsrc, int* flag, float* out) {
-  gj_panels<float, 16, 1, 16>(c, n, a, b, d, prm, rowsrc, flag, out);
+constexpr int kGjWidth32 = 16, kGjWidth64 = 8;
+static void gj_inverse(pm_ctx* c, int n, float* work, int* prm, int* rowsrc, int* flag, float* out) {
+  gj_panels<float, kGjWidth32, 1, 16>(c, n, work, prm, rowsrc, flag, out);
 }
-static void gj_inverse(pm_ctx* c, int n, double* a, double* b, double* d, int* prm, int* rowsrc, int* flag,
-                       double* out) {
-  gj_panels<double, 8, 4, 16>(c, n, a, b, d, prm, rowsrc, flag, out);
+static void gj_inverse(pm_ctx* c, int n, double* work, int* prm, int* rowsrc, int* flag, double* out) {
+  gj_panels<double, kGjWidth64, 4, 16>(c, n, work, prm, rowsrc, flag, out);
 }
 
 __global__ void k_coarse_gemv32(int n, int na, const int* __restrict__ act, const int* __restrict__ pos,
@@ -1417,9 +1425,9 @@ void DenseInverse::launch32(pm_ctx* c, const DevCsr& A, cudaStream_t s) {
   StreamSwap swap(c, s);
   const size_t nn = size_t(na) * na;
   inv32.ensure(nn);
-  work32.ensure(2 * nn + 2 * 16 * 16);
-  prepare(c, A, work32.p);
-  gj_inverse(c, na, work32.p, work32.p + nn, work32.p + 2 * nn, perm.p, perm.p + na, flag.p, inv32.p);
+  work32.ensure(nn + 2 * kGjWidth32 * kGjWidth32);
+  prepare(c, A, gj_start(na, kGjWidth32, work32.p, inv32.p));
+  gj_inverse(c, na, work32.p, perm.p, perm.p + na, flag.p, inv32.p);
   if (!done_event) PM_CUDA(cudaEventCreateWithFlags(&done_event, cudaEventDisableTiming));
   PM_CUDA(cudaEventRecord(done_event, s));
   pending32 = true;
@@ -1521,9 +1529,9 @@ void DenseInverse::launch64(pm_ctx* c, const DevCsr& A, cudaStream_t s) {
   inv.ensure(nn);
   const bool panels = na <= kGjMaxRows;
   if (panels && na) {
-    work.ensure(2 * nn + 2 * 8 * 8);
-    prepare(c, A, work.p);
-    gj_inverse(c, na, work.p, work.p + nn, work.p + 2 * nn, perm.p, perm.p + na, flag.p, inv.p);
+    work.ensure(nn + 2 * kGjWidth64 * kGjWidth64);
+    prepare(c, A, gj_start(na, kGjWidth64, work.p, inv.p));
+    gj_inverse(c, na, work.p, perm.p, perm.p + na, flag.p, inv.p);
   } else {
     prepare(c, A, inv.p);
     if (na == 0) {

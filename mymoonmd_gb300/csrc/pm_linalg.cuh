@@ -177,7 +177,7 @@ struct DenseInverse {
   DBuf<int> flag;    // singular pivot flag
   DBuf<double> rowk, oldk, part_v;  // column-by-column elimination: pivot row, old row k, block arg-max
   DBuf<int> part_i;
-  // blocked elimination: the matrix before and after a panel, the panel
+  // blocked elimination: the matrix beside inv (before or after a panel), the panel
   DBuf<double> work;
   DBuf<float> work32;
   BlockMask rows_of{};   // the block layout act / pos were made for
