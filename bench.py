@@ -436,7 +436,7 @@ def run_ours(args, w, rank, world, local, pg):
 
 
 PROBE_EPILOGUE = 3  # EPI_JACOBI (include/pmgpu.h, probe_epilogue)
-SLICED_DEFAULT = 481  # the library's default fp32_sliced_spmv shape
+SLICED_DEFAULT = 482  # the library's default fp32_sliced_spmv shape
 
 
 def profiled_traffic(wname):

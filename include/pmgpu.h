@@ -79,10 +79,11 @@ int pm_version(void);
  *   copies' values are refreshed with the Vanka factors;
  *   "fp32_sliced_spmv" 0|100 L + 10 U + P - FP32 SpMV-family launches on
  *   matrices with more than 16 entries per row by the sliced-ELL kernel: L
- *   lanes per row (1, 2, 4, 8), U steps in flight (4, 8; 481 keeps sixteen),
- *   P = 1 issues the next steps' loads before the current gathers; accepted: 140 141 180 240 241 280
- *   440 441 480 481 840 841 881; 0 = the row-group kernel on the CSR arrays.
- *   Default 481. The sliced copy (rows sorted by length in windows of 1024,
+ *   lanes per row (1, 2, 4, 8), U steps in flight (4, 8), P = 1 issues the next
+ *   steps' loads before the current gathers, P = 2 that with 2 U steps in flight on
+ *   matrices of long rows and few slices; accepted: 140 141 180 240 241 280 440 441
+ *   480 481 482 840 841 881; 0 = the row-group kernel on the CSR arrays.
+ *   Default 482. The sliced copy (rows sorted by length in windows of 1024,
  *   slices of 32/L rows, padded to the slice's longest row) is laid out when
  *   the FP32 values are made (pm_matrix_make_fp32, the multigrid update) for
  *   the shape's L. Shapes with the same L give the same bits;
@@ -90,9 +91,8 @@ int pm_version(void);
  *   cycle, of the row-group sweeps with programmatic stream serialization (a sweep loads its slice layout and first values while the
  *   previous kernel finishes, and waits for it before reading vectors; default
  *   1: on GB300 the 3D Q2 request took 26.9 ms with 1, 27.6 ms with 0);
- *   "fp64_sliced_spmv" 0|441|481|841 - the same for FP64 values (the Krylov
- *   SpMV, the FP64 multigrid); used when its L equals the layout's (default 441,
- *   which keeps eight steps in flight on matrices of at most 128 slices per SM);
+ *   "fp64_sliced_spmv" 0|441|442|481|841 - the same for FP64 values (the Krylov
+ *   SpMV, the FP64 multigrid); used when its L equals the layout's (default 442);
  *   "jacobi_zero_start" 0|1 - the first damped Jacobi sweep of a multigrid level
  *   whose iterate is exactly zero (coarse levels after their reset; the finest
  *   level inside FGMRES when the initial residual has zero non-actives) as the

@@ -76,16 +76,16 @@ int pm_ctx_set_option(pm_ctx* c, const char* key, int value) {
     return PM_OK;
   }
   if (std::string(key) == "fp32_sliced_spmv") {
-    static const int shapes[] = {0, 140, 141, 180, 240, 241, 280, 440, 441, 480, 481, 840, 841, 881};
+    static const int shapes[] = {0, 140, 141, 180, 240, 241, 280, 440, 441, 480, 481, 482, 840, 841, 881};
     if (std::find(std::begin(shapes), std::end(shapes), value) == std::end(shapes))
       return fail(c, PM_E_INVALID,
-                  "fp32_sliced_spmv is 0 or one of 140 141 180 240 241 280 440 441 480 481 840 841 881");
+                  "fp32_sliced_spmv is 0 or one of 140 141 180 240 241 280 440 441 480 481 482 840 841 881");
     c->sell_shape = value;
     return PM_OK;
   }
   if (std::string(key) == "fp64_sliced_spmv") {
-    if (value != 0 && value != 441 && value != 481 && value != 841)
-      return fail(c, PM_E_INVALID, "fp64_sliced_spmv is 0, 441, 481 or 841");
+    if (value != 0 && value != 441 && value != 442 && value != 481 && value != 841)
+      return fail(c, PM_E_INVALID, "fp64_sliced_spmv is 0, 441, 442, 481 or 841");
     c->sell_shape64 = value;
     return PM_OK;
   }

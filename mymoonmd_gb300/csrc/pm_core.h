@@ -114,12 +114,12 @@ struct pm_ctx {
   const int* guard = nullptr;
   // FP32 SpMV by the sliced-ELL kernel: 0 = off, else 100 L + 10 U + P (L lanes
   // per row, U steps in flight, P = 1: next steps' loads issued before the
-  // current gathers); the matrix copies are laid out for L in make_fp32. 481
-  // keeps sixteen steps in flight, 441 for FP64 eight on small matrices
-  int sell_shape = 481;
+  // current gathers; P = 2: that, with 2 U steps in flight on small matrices); the
+  // matrix copies are laid out for L in make_fp32
+  int sell_shape = 482;
   // FP64 SpMV-family launches by the sliced-ELL kernel (same encoding; the
   // layout's lanes must equal those of the FP32 shape when both are used)
-  int sell_shape64 = 441;
+  int sell_shape64 = 442;
   // matrices with more entries per row than this on average get sliced copies
   // (option "sliced_min_entries")
   int sell_min_avg = 16;

@@ -456,11 +456,25 @@ static void launch_sell_shape(pm_ctx* c, const DevCsr& A, int epi, const T* x, T
   }
 }
 
-// FP64 shape 441 on matrices of few slices: eight steps in flight instead of four
-// (the sums are the same). At most 128 slices per SM, FP64 cycle of 3D Q2 in us,
-// four / eight: 16^3 (36 slices per SM in the finest sweep) 129 / 105, 24^3 (97)
-// 235 / 220, 28^3 (152) 263 / 271, 32^3 (226) 378 / 378 with the SpMV 39.2 / 42.8
-static bool sell_deep(const pm_ctx* c, long long n_slices) { return n_slices <= 128ll * c->num_sms; }
+// Shapes 442 (FP64) and 482 (FP32): twice the steps in flight where rows are longer
+// than eight steps on average and a launch has few slices (the sums are the same). Four lanes, half / twice the steps:
+//   FP64 cycle of 3D Q2 in us: 8^3 49.9 / 43.8, 16^3 135.6 / 101.9 (30 slices per SM
+//   in the finest sweep), 24^3 211.5 / 195.9 (97); above 128 slices per SM the finest
+//   sweep is no faster (28^3 263 / 271, the SpMV of 32^3 39.2 / 42.8). Product of the
+//   combined Stokes matrix of 12^3 20.2 / 13.0.
+//   FP32 cycle of 3D Q2: 8^3 31.0 / 29.1, 16^3 61.5 / 56.0, 24^3 105.3 / 103.0; the
+//   finest sweep of 32^3 (226) 28.8 / 28.9.
+//   Short rows (3D Q1: at most seven steps) lose: FP32 cycle of 32^3 48.3 / 51.3, 48^3
+//   66.6 / 76.1; FP64 32^3 88.1 / 89.5, 48^3 127.2 / 140.8. Only FP64 launches of few
+//   slices gain (16^3, 4 slices per SM: 53.1 / 49.4).
+static bool sell_long_rows(const DevCsr& A) { return A.sell_entries > 8ll * 32 * A.n_slices; }
+static bool sell_deep64(const pm_ctx* c, const DevCsr& A, int ns = 1) {
+  const long long slices = (long long)A.n_slices * ns;
+  return slices <= (sell_long_rows(A) ? 128ll : 16ll) * c->num_sms;
+}
+static bool sell_deep32(const pm_ctx* c, const DevCsr& A, int ns = 1) {
+  return sell_long_rows(A) && (long long)A.n_slices * ns <= 128ll * c->num_sms;
+}
 
 static void launch_sell(pm_ctx* c, const DevCsr& A, int epi, const float* x, float* y, const float* b,
                         const float* d, float alpha) {
@@ -476,9 +490,11 @@ static void launch_sell(pm_ctx* c, const DevCsr& A, int epi, const float* x, flo
     case 440: launch_sell_shape<float, 4, 4, false>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 441: launch_sell_shape<float, 4, 4, true>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 480: launch_sell_shape<float, 4, 8, false>(c, A, epi, x, y, b, d, alpha, mg); break;
-    // sixteen steps in flight: mixed cycle of 3D Q2 in us, eight / sixteen: 8^3
-    // 41.9 / 38.3, 16^3 63.9 / 57.5, 24^3 122.5 / 115.4, 32^3 194 / 190
-    case 481: launch_sell_shape<float, 4, 16, true>(c, A, epi, x, y, b, d, alpha, mg); break;
+    case 481: launch_sell_shape<float, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg); break;
+    case 482:
+      if (sell_deep32(c, A)) launch_sell_shape<float, 4, 16, true>(c, A, epi, x, y, b, d, alpha, mg);
+      else launch_sell_shape<float, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg);
+      break;
     case 840: launch_sell_shape<float, 8, 4, false>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 841: launch_sell_shape<float, 8, 4, true>(c, A, epi, x, y, b, d, alpha, mg); break;
     case 881: launch_sell_shape<float, 8, 8, true>(c, A, epi, x, y, b, d, alpha, mg); break;
@@ -493,8 +509,9 @@ static void launch_sell64(pm_ctx* c, const DevCsr& A, int epi, const double* x, 
   BlockMask mg = A.mask;
   mg.guard = c->guard;
   switch (c->sell_shape64) {
-    case 441:
-      if (sell_deep(c, A.n_slices)) launch_sell_shape<double, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg);
+    case 441: launch_sell_shape<double, 4, 4, true>(c, A, epi, x, y, b, d, alpha, mg); break;
+    case 442:
+      if (sell_deep64(c, A)) launch_sell_shape<double, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg);
       else launch_sell_shape<double, 4, 4, true>(c, A, epi, x, y, b, d, alpha, mg);
       break;
     case 481: launch_sell_shape<double, 4, 8, true>(c, A, epi, x, y, b, d, alpha, mg); break;
@@ -1749,8 +1766,9 @@ void csr_apply_batch(pm_ctx* c, const DevCsr& A, int ns, const Batch& bt, int ep
   if (A.stream && A.n_rblocks > 0) throw Error(PM_E_UNSUPPORTED, "batched launch of the streaming CSR kernel");
   if (c->sell_shape64 > 0 && A.sell64_ok && A.sell_lanes == c->sell_shape64 / 100 && A.n_slices > 0) {
     switch (c->sell_shape64) {
-      case 441:
-        if (sell_deep(c, (long long)A.n_slices * ns)) launch_sell_batch<double, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask);
+      case 441: launch_sell_batch<double, 4, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask); break;
+      case 442:
+        if (sell_deep64(c, A, ns)) launch_sell_batch<double, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask);
         else launch_sell_batch<double, 4, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask);
         break;
       case 481: launch_sell_batch<double, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag.p, alpha, A.mask); break;
@@ -1771,7 +1789,11 @@ void csr_apply32_batch(pm_ctx* c, const DevCsr& A, int ns, const Batch& bt, int 
   if (c->sell_shape > 0 && A.sell_lanes == c->sell_shape / 100 && A.n_slices > 0) {
     switch (c->sell_shape) {
       case 441: launch_sell_batch<float, 4, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
-      case 481: launch_sell_batch<float, 4, 16, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
+      case 481: launch_sell_batch<float, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
+      case 482:
+        if (sell_deep32(c, A, ns)) launch_sell_batch<float, 4, 16, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask);
+        else launch_sell_batch<float, 4, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask);
+        break;
       case 841: launch_sell_batch<float, 8, 4, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
       case 881: launch_sell_batch<float, 8, 8, true>(c, A, ns, bt, epi, x, y, b, A.diag32.p, alpha, A.mask); break;
       default: throw Error(PM_E_UNSUPPORTED, "batched launch of sliced shape " + std::to_string(c->sell_shape));
