@@ -68,14 +68,15 @@ int pm_version(void);
  *   4 restriction, 5 prolongation add; -1 = all);
  *   "probe_precision" 0|4|8 - only launches whose matrix values have this
  *   size in bytes (0 = all);
- *   "probe_nodal" 0|1 - the launch probe brackets instead the residual and
- *   local-solve pair of every colour of the multiplicative nodal Vanka
- *   sweeps (counted as one launch, with the pair's algorithmic bytes);
+ *   "probe_nodal" 0|1 - the launch probe brackets instead every colour of the
+ *   multiplicative nodal Vanka sweeps (its kernel, or its residual and
+ *   local-solve pair, counted as one launch, with the algorithmic bytes);
  *   "nodal_sliced" 0|4|8 - nodal Vanka sweeps by one kernel per colour over
  *   packed patches (8, default; packed when a problem sets up its smoothers, up
- *   to 32 colours; a matrix whose velocity blocks differ is swept as with 0), or with the local residuals of a colour by one sliced-ELL
- *   launch over a copy of its patches' rows (4, 1 = 4; also 8 where the patches
- *   do not fit the kernel) or by one block per patch over the CSR rows (0); the
+ *   to 32 colours; a matrix whose velocity blocks differ is swept as with 0), or
+ *   with the local residuals of a colour by one sliced-ELL launch over a copy of
+ *   its patches' rows, four lanes per row (4, 1 = 4; also 8 where the patches do
+ *   not fit the kernel) or by one block per patch over the CSR rows (0); the
  *   copies' values are refreshed with the Vanka factors;
  *   "fp32_sliced_spmv" 0|100 L + 10 U + P - FP32 SpMV-family launches on
  *   matrices with more than 16 entries per row by the sliced-ELL kernel: L

@@ -139,7 +139,7 @@ struct pm_ctx {
   // residual + local-solve pair of every colour (option "probe_nodal")
   int probe_nodal = 0;
   // nodal Vanka sweeps: 8 = one kernel per colour over packed patches where they
-  // fit it (else as 4 with 8 lanes per row), 4 = local residuals from a
+  // fit it (else as 4), 4 = local residuals from a
   // per-colour sliced copy of the patch rows, 0 = from the CSR rows, one block
   // per patch (option "nodal_sliced"; read when a problem lays out its smoothers)
   int nodal_sliced = 8;

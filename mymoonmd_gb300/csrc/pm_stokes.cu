@@ -982,8 +982,7 @@ namespace pm {
 void DevNodalVanka::build_row_slices(pm_ctx* c, const pmsetup::Csr& S, int p0, const std::vector<int>& vp,
                                      const std::vector<int>& vi, const std::vector<int>& cp) {
   rs_ok = false;
-  rs_lanes = 0;
-  const int Lanes = c->nodal_sliced == 8 ? 8 : 4, C = 32 / Lanes;
+  constexpr int Lanes = 4, C = 32 / Lanes;
   if (c->nodal_sliced == 0) return;
   // the projected structure: row p0 holds only its diagonal
   auto row_len = [&](int g) { return g == p0 ? 1 : S.row_ptr[g + 1] - S.row_ptr[g]; };
@@ -1053,7 +1052,6 @@ void DevNodalVanka::build_row_slices(pm_ctx* c, const pmsetup::Csr& S, int p0, c
   bslot.upload(slot_row, c->stream);
   PM_CUDA(cudaStreamSynchronize(c->stream));  // the host vectors go out of scope
   rs_entries = total;
-  rs_lanes = Lanes;
   rs_ok = true;
 }
 
@@ -2479,12 +2477,8 @@ static bool nodal_colored(pm_ctx* c, DevNodalVanka& nv, const DevCsr& V, const T
     if (sliced) {
       // the colour's local residuals as one sliced SpMV: rloc[slot] = bloc[slot] - (V x)[row]
       const int s0 = nv.color_slice[k], ns = nv.color_slice[k + 1] - s0;
-      if (nv.rs_lanes == 8)
-        sell_kernel<T, 8, 8, true, EPI_DEFECT><<<(ns + 3) / 4, 128, 0, c->stream>>>(
-            ns, nv.rs_perm.p + size_t(s0) * 4, nv.rs_off.p + s0, nv.rs_cols.p, rsv, x, rloc, bl, nullptr, T(0), mg);
-      else
-        sell_kernel<T, 4, 8, true, EPI_DEFECT><<<(ns + 3) / 4, 128, 0, c->stream>>>(
-            ns, nv.rs_perm.p + size_t(s0) * 8, nv.rs_off.p + s0, nv.rs_cols.p, rsv, x, rloc, bl, nullptr, T(0), mg);
+      sell_kernel<T, 4, 8, true, EPI_DEFECT><<<(ns + 3) / 4, 128, 0, c->stream>>>(
+          ns, nv.rs_perm.p + size_t(s0) * 8, nv.rs_off.p + s0, nv.rs_cols.p, rsv, x, rloc, bl, nullptr, T(0), mg);
     } else {
       k_nodal_rhs<T><<<cnt, 512, 0, c->stream>>>(c->guard, cnt, pts, nv.nu, nv.vptr.p, nv.vidx.p, V.row_ptr.p,
                                                   V.cols.p, vals, b, x, rloc);

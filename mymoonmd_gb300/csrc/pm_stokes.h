@@ -170,7 +170,6 @@ struct DevNodalVanka {
   // Slices of colour k: color_slice[k] .. color_slice[k+1]. bslot: the global
   // row of each slot (the smoother's right-hand side gathered once per sweep)
   bool rs_ok = false;
-  int rs_lanes = 0;  // lanes per row of the copy (4 or 8)
   std::vector<int> color_slice;
   int64_t rs_entries = 0;
   DBuf<int> rs_perm, rs_off, rs_cols, rs_src, bslot;
