@@ -75,12 +75,12 @@ __global__ void k_heads(long long total, int n, const unsigned long long* __rest
   }
 }
 
-// CSR columns, row starts, gather plan and the non-active diagonals
-__global__ void k_fill_structure(long long total, int n, int n_active, const unsigned long long* __restrict__ key,
+// CSR columns, row starts and gather plan
+__global__ void k_fill_structure(long long total, int n, const unsigned long long* __restrict__ key,
                                  const int* __restrict__ val, const int* __restrict__ head,
                                  const int* __restrict__ hpos, const int* __restrict__ cpos,
                                  int* __restrict__ row_ptr, int* __restrict__ cols, int* __restrict__ gat_ptr,
-                                 int* __restrict__ gat_idx, int* __restrict__ diag_pos) {
+                                 int* __restrict__ gat_idx) {
   const unsigned long long invalid = (unsigned long long)n * n;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -92,7 +92,6 @@ __global__ void k_fill_structure(long long total, int n, int n_active, const uns
       cols[p] = int(k % n);
       gat_ptr[p] = cpos[i];
       if (i == 0 || int(key[i - 1] / n) != row) row_ptr[row] = p;
-      if (val[i] < 0) diag_pos[row - n_active] = p;
     }
     if (val[i] >= 0) gat_idx[cpos[i]] = val[i];
   }
@@ -334,31 +333,6 @@ __global__ void k_stokes_pairs(int n_cells, int N, int n_inactive, const int* __
   }
 }
 
-// as k_fill_structure, with the non-active rows' diagonal positions indexed
-// by their rank among the non-active rows
-__global__ void k_fill_structure_ranked(long long total, int n, const unsigned long long* __restrict__ key,
-                                        const int* __restrict__ val, const int* __restrict__ head,
-                                        const int* __restrict__ hpos, const int* __restrict__ cpos,
-                                        const int* __restrict__ inactive_rank, int* __restrict__ row_ptr,
-                                        int* __restrict__ cols, int* __restrict__ gat_ptr, int* __restrict__ gat_idx,
-                                        int* __restrict__ diag_pos) {
-  const unsigned long long invalid = (unsigned long long)n * n;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = key[i];
-    if (k >= invalid) continue;
-    const int row = int(k / n);
-    if (head[i]) {
-      const int p = hpos[i];
-      cols[p] = int(k % n);
-      gat_ptr[p] = cpos[i];
-      if (i == 0 || int(key[i - 1] / n) != row) row_ptr[row] = p;
-      if (val[i] < 0) diag_pos[inactive_rank[row]] = p;
-    }
-    if (val[i] >= 0) gat_idx[cpos[i]] = val[i];
-  }
-}
-
 // right-hand side items t = c * 34 + m: key = row for active rows, N otherwise
 __global__ void k_stokes_rhs_pairs(long long nt, int N, const int* __restrict__ cdof,
                                    const unsigned char* __restrict__ act, unsigned int* __restrict__ key,
@@ -429,9 +403,8 @@ void device_level_structure(pm_ctx* c, DiscLevel& L) {
   const int nnz = last[0] + last[1], ncontrib = last[2] + last[3];
   DBuf<int> row_ptr(static_cast<size_t>(n) + 1), cols(static_cast<size_t>(nnz));
   DBuf<int> gat_ptr(static_cast<size_t>(nnz) + 1), gat_idx(static_cast<size_t>(ncontrib));
-  DBuf<int> diag_pos(static_cast<size_t>(std::max(1, n - na)));
-  k_fill_structure<<<grid, 256, 0, st>>>(total, n, na, key_out.p, val_out.p, head.p, hpos.p, cpos.p, row_ptr.p,
-                                         cols.p, gat_ptr.p, gat_idx.p, diag_pos.p);
+  k_fill_structure<<<grid, 256, 0, st>>>(total, n, key_out.p, val_out.p, head.p, hpos.p, cpos.p, row_ptr.p,
+                                         cols.p, gat_ptr.p, gat_idx.p);
   PM_CHECK_LAUNCH();
   k_set_tail<<<1, 32, 0, st>>>(row_ptr.p, n, n + 1, nnz);
   k_set_tail<<<1, 32, 0, st>>>(gat_ptr.p, nnz, nnz + 1, ncontrib);
@@ -467,7 +440,6 @@ void device_level_structure(pm_ctx* c, DiscLevel& L) {
   download(c, L.sys.cols, cols, size_t(nnz));
   download(c, L.gat_ptr, gat_ptr, size_t(nnz) + 1);
   download(c, L.gat_idx, gat_idx, size_t(ncontrib));
-  download(c, L.diag_pos, diag_pos, size_t(n - na));
   // the items of non-active DOFs sort last: the valid count is the number of
   // positions t whose DOF is active
   long long valid = 0;
@@ -613,12 +585,9 @@ void device_stokes_structure(pm_ctx* c, DiscLevel& L, const std::vector<char>& a
     S.lk[j] = short(loc.k[j]);
     S.lpos[j] = short(loc.pos[j]);
   }
-  std::vector<int> inactive, rank(N, -1);
+  std::vector<int> inactive;
   for (int i = 0; i < N; ++i)
-    if (!active[i]) {
-      rank[i] = int(inactive.size());
-      inactive.push_back(i);
-    }
+    if (!active[i]) inactive.push_back(i);
   const int ni = int(inactive.size()), na = N - ni;
   const long long ne = (long long)nc * S.n, total = ne + ni;
   const long long nt = (long long)nc * 34;
@@ -626,13 +595,12 @@ void device_stokes_structure(pm_ctx* c, DiscLevel& L, const std::vector<char>& a
     throw Error(PM_E_INVALID, "level too large for the device structure build");
   const int grid = std::max(1, std::min(int((total + 255) / 256), c->num_sms * 8));
   cudaStream_t st = c->stream;
-  DBuf<int> cdof, inact, irank;
+  DBuf<int> cdof, inact;
   DBuf<unsigned char> act;
   cdof.upload(L.cdof, st);
   std::vector<unsigned char> a8(active.begin(), active.end());
   act.upload(a8, st);
   inact.upload(inactive.empty() ? std::vector<int>{0} : inactive, st);
-  irank.upload(rank, st);
   DBuf<unsigned long long> key_in(static_cast<size_t>(total)), key_out(static_cast<size_t>(total));
   DBuf<int> val_in(static_cast<size_t>(total)), val_out(static_cast<size_t>(total));
   k_stokes_pairs<<<grid, 256, 0, st>>>(nc, N, ni, cdof.p, act.p, inact.p, S, key_in.p, val_in.p);
@@ -663,9 +631,8 @@ void device_stokes_structure(pm_ctx* c, DiscLevel& L, const std::vector<char>& a
   const int nnz = last[0] + last[1], ncontrib = last[2] + last[3];
   DBuf<int> row_ptr(static_cast<size_t>(N) + 1), cols(static_cast<size_t>(nnz));
   DBuf<int> gat_ptr(static_cast<size_t>(nnz) + 1), gat_idx(static_cast<size_t>(std::max(1, ncontrib)));
-  DBuf<int> diag_pos(static_cast<size_t>(std::max(1, ni)));
-  k_fill_structure_ranked<<<grid, 256, 0, st>>>(total, N, key_out.p, val_out.p, head.p, hpos.p, cpos.p, irank.p,
-                                                row_ptr.p, cols.p, gat_ptr.p, gat_idx.p, diag_pos.p);
+  k_fill_structure<<<grid, 256, 0, st>>>(total, N, key_out.p, val_out.p, head.p, hpos.p, cpos.p, row_ptr.p, cols.p,
+                                         gat_ptr.p, gat_idx.p);
   PM_CHECK_LAUNCH();
   k_set_tail<<<1, 32, 0, st>>>(row_ptr.p, N, N + 1, nnz);
   k_set_tail<<<1, 32, 0, st>>>(gat_ptr.p, nnz, nnz + 1, ncontrib);
@@ -695,7 +662,6 @@ void device_stokes_structure(pm_ctx* c, DiscLevel& L, const std::vector<char>& a
   download(c, L.sys.cols, cols, size_t(nnz));
   download(c, L.gat_ptr, gat_ptr, size_t(nnz) + 1);
   download(c, L.gat_idx, gat_idx, size_t(ncontrib));
-  download(c, L.diag_pos, diag_pos, size_t(ni));
   std::vector<unsigned> rk(static_cast<size_t>(nt));
   std::vector<int> rv;
   download(c, rv, rval_out, size_t(nt));

@@ -6,7 +6,7 @@
 namespace pm {
 
 // L.sys (the square CSR structure of L.space), the assembly gather plans
-// gat_ptr / gat_idx and rgat_ptr / rgat_idx, and diag_pos, built on the
+// gat_ptr / gat_idx and rgat_ptr / rgat_idx, built on the
 // context's GPU by sorting and copied into L: the same arrays as the host
 // construction of build_disc.
 void device_level_structure(pm_ctx* c, DiscLevel& L);

@@ -54,10 +54,6 @@ static void build_gather(DiscLevel& L, int nloc, const std::vector<int>& gdof,
   std::vector<int> rf(rc.begin(), rc.end() - 1);
   for (size_t t = 0; t < gdof.size(); ++t)
     if (row_active[gdof[t]]) L.rgat_idx[rf[gdof[t]]++] = int(t);
-  // unit diagonal of non-active rows
-  L.diag_pos.clear();
-  for (int i = 0; i < n; ++i)
-    if (!row_active[i]) L.diag_pos.push_back(find(i, i));
 }
 
 // --------------------------------------------------------------- Stokes ----
@@ -223,9 +219,6 @@ static void build_stokes_structure(DiscLevel& L, const std::vector<char>& act) {
     for (size_t t = 0; t < L.cdof.size(); ++t)
       if (act[L.cdof[t]]) L.rgat_idx[fill[L.cdof[t]]++] = int(t);  // rhs storage: cell*34 + m
   }
-  L.diag_pos.clear();
-  for (int i = 0; i < N; ++i)
-    if (!act[i]) L.diag_pos.push_back(find(i, i));
 }
 
 // block layout, Vanka patches and the cell colouring of a Stokes level

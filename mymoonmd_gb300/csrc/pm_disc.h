@@ -21,12 +21,11 @@ struct DiscLevel {
   std::vector<double> verts;  // cell vertex coordinates
   // assembly gather plan: for each CSR entry of an active row, the positions
   // (cell * nloc * nloc + m * nloc + k) of the element-matrix entries that add
-  // to it, in cell order (the order Assemble3D.C:346-370 adds them)
+  // to it, in cell order (the order Assemble3D.C:346-370 adds them); an entry of a
+  // non-active row, its diagonal, has none
   std::vector<int> gat_ptr, gat_idx;
   // right-hand side gather plan: for each active DOF, positions cell*nloc + m
   std::vector<int> rgat_ptr, rgat_idx;
-  // Dirichlet rows: CSR position of the diagonal entry
-  std::vector<int> diag_pos;
   // physical coordinates (x, y, z; z = 0 in 2D) of the non-active DOFs
   // n_active .. n_dofs-1 of `space` (for Stokes the velocity component space),
   // the points of the nodal functionals the Dirichlet values are taken at
@@ -69,14 +68,14 @@ struct Disc {
 // pm_devsetup.cu); each gives the same arrays as the host construction it
 // replaces. hierarchy: the mesh hierarchy (build_hierarchy); space: a level's
 // numbering (build_space); structure: a convection-diffusion level's `sys`,
-// gather plans and diag_pos from its space.
+// gather plans from its space.
 struct SetupParts {
   std::function<pmsetup::Hierarchy(int geometry, int root_n, int n_refine)> hierarchy;
   std::function<pmsetup::Space(const pmsetup::Hierarchy&, int level, int elem, int boundary, int neumann_sides)>
       space;
   std::function<void(DiscLevel&)> structure;
-  // a Stokes level's combined `sys`, gather plans and diag_pos from its cdof
-  // and the active flags of the combined DOFs
+  // a Stokes level's combined `sys` and gather plans from its cdof and the
+  // active flags of the combined DOFs
   std::function<void(DiscLevel&, const std::vector<char>& active)> stokes_structure;
 };
 

@@ -41,13 +41,6 @@ void ctx_destroy(pm_ctx* c) {
 static inline int nblocks(long long n, int t) { return int((n + t - 1) / t); }
 
 // -------------------------------------------------------------------- CSR ---
-int choose_lanes(double avg) {
-  if (avg <= 6.0) return 4;
-  if (avg <= 12.0) return 8;
-  if (avg <= 28.0) return 16;
-  return 32;
-}
-
 void DevCsr::upload(pm_ctx* c, int nr, int nc, int na, const int* rp, const int* ci,
                     const double* v) {
   n_rows = nr;
@@ -761,15 +754,9 @@ void nonactive_nonzero(pm_ctx* c, const BlockMask& m, const double* x, int* flag
   c->kernel_launches++;
 }
 
-// x = 0 + w ((b - 0) / d): the damped Jacobi sweep of an exactly zero iterate
-// (the sweep's row sums of a_ij * 0 are +0; fma(w, q, +0) rounds like its
-// x + w q with x = +0)
-template <class T>
-__global__ void k_jacobi_zero(int n, const T* __restrict__ b, const T* __restrict__ d, T w, T* __restrict__ x) {
-  pdl_enter();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    x[i] = fmadd(w, (b[i] - T(0)) / d[i], T(0));
-}
+// x = 0 + w ((b - 0) / d) is the damped Jacobi sweep of an exactly zero iterate (the
+// sweep's row sums of a_ij * 0 are +0; fma(w, q, +0) rounds like its x + w q with
+// x = +0).
 // set_finest_rhs and the first step of the cycle in one launch (a conversion, an
 // initialisation and, from zero, a diagonal scaling were three)
 template <class T>
@@ -790,13 +777,6 @@ template void cycle_start<float>(pm_ctx*, int, const BlockMask&, const double*, 
                                  bool);
 template void cycle_start<double>(pm_ctx*, int, const BlockMask&, const double*, double*, double*, const double*,
                                   double, bool);
-void jacobi_from_zero(pm_ctx* c, int n, const double* b, const double* d, double w, double* x) {
-  PM_LAUNCH1D(k_jacobi_zero<double>, n, n, b, d, w, x);
-}
-void jacobi_from_zero32(pm_ctx* c, int n, const float* b, const float* d, float w, float* x) {
-  PM_LAUNCH1D(k_jacobi_zero<float>, n, n, b, d, w, x);
-}
-
 // ------------------------------------------------------------ SOR ----------
 void SorColours::build(pm_ctx* c, const DevCsr& A) {
   if (key == A.row_ptr.p && key_nnz == A.nnz) return;

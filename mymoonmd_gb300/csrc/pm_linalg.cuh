@@ -88,7 +88,6 @@ struct DevCsr {
   size_t spmv_bytes(int elem_bytes, bool read_y) const;
 };
 
-int choose_lanes(double avg_nnz_per_row);
 constexpr int kStreamNnz = 2048;  // entries per row block of the streaming kernel
 // greedy row blocks over a host row-pointer array; empty if a row is too long
 std::vector<int> build_row_blocks(int n_rows, const int* rp, int max_nnz, int max_rows);
@@ -131,9 +130,6 @@ void vaxpy(pm_ctx* c, int n, double a, const double* x, double* y);  // y += a x
 void vaxpby(pm_ctx* c, int n, double a, const double* x, double b, double* y);  // y = a x + b y
 void vcvt_d2f(pm_ctx* c, int n, const double* x, float* y);
 void vcvt_f2d(pm_ctx* c, int n, const float* x, double* y);
-// x := w (b / d), the damped Jacobi sweep from x = 0
-void jacobi_from_zero(pm_ctx* c, int n, const double* b, const double* d, double w, double* x);
-void jacobi_from_zero32(pm_ctx* c, int n, const float* b, const float* d, float w, float* x);
 void vdiv(pm_ctx* c, int n, const double* d, double* y);  // y /= d
 // BlockVector::copy_nonactive: dst := src on the non-active rows
 void copy_nonactive(pm_ctx* c, int n, const BlockMask& m, const double* src, double* dst);

@@ -269,19 +269,6 @@ void Multigrid::smooth(pm_ctx* c, int l) {
   }
 }
 
-void Multigrid::smooth_from_zero(pm_ctx* c, int l) {
-  MGLevel& lv = levels[l];
-  const DevCsr& A = lv.A->csr;
-  if (lv.smoother != SM_JACOBI || !c->jacobi_zero_start) {
-    smooth(c, l);
-    return;
-  }
-  // the iterate stays in its buffer (the sweep's swap of the two buffers is
-  // not needed: x0 is not read)
-  if (mixed) jacobi_from_zero32(c, A.n_rows, lv.rhs32.p, A.diag32.p, float(jacobi_damp), lv.cur32);
-  else jacobi_from_zero(c, A.n_rows, lv.rhs.p, A.diag.p, jacobi_damp, lv.cur);
-}
-
 void Multigrid::coarse_solve(pm_ctx* c) {
   MGLevel& lv = levels[0];
   const DevCsr& A = lv.A->csr;
@@ -453,12 +440,10 @@ void Multigrid::apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonact
     explicit InCycle(pm_ctx* c_) : c(c_) { c->in_cycle = true; }
     ~InCycle() { c->in_cycle = false; }
   } in_cycle(c);
-  // levels whose iterate is exactly zero now: the finest one when its rhs has
-  // zero non-actives (init_solution copies them), the coarser ones after their
-  // reset below (their rhs has its non-actives reset by the restriction)
-  // swept: the level's first sweep from zero has been done with its right-hand side
-  std::vector<char> zero(L, 0), swept(L, 0);
-  zero[finest] = rhs_nonactive_zero ? 1 : 0;
+  // levels whose first pre-smoothing sweep, from an iterate that is exactly zero, came
+  // with their right-hand side: the finest one when its rhs has zero non-actives, the
+  // coarser ones with their restriction (which resets the non-actives)
+  std::vector<char> swept(L, 0);
   swept[finest] = top_swept ? 1 : 0;
   const int n_steps = int(control.size()) - 1;
   int level = finest;
@@ -468,9 +453,7 @@ void Multigrid::apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonact
       // the defects the reference computes around it only feed its loop test
       if (levels[0].smoother == SM_DIRECT) coarse_solve(c);
       else coarse_iterate(c);
-      zero[0] = 0;
       prolongate_from(c, 0);
-      zero[1] = 0;
       level = 1;
       continue;
     }
@@ -482,9 +465,7 @@ void Multigrid::apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonact
     if (down) {
       for (int i = 0; i < n_pre; ++i) {
         if (i == 0 && swept[level]) swept[level] = 0;
-        else if (i == 0 && zero[level]) smooth_from_zero(c, level);
         else smooth(c, level);
-        zero[level] = 0;
       }
       defect(c, level);
       MGLevel& crs = levels[level - 1];
@@ -498,13 +479,11 @@ void Multigrid::apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonact
         if (mixed) PM_CUDA(cudaMemsetAsync(crs.cur32, 0, sizeof(float) * nc, c->stream));
         else PM_CUDA(cudaMemsetAsync(crs.cur, 0, sizeof(double) * nc, c->stream));
       }
-      zero[level - 1] = 1;
       swept[level - 1] = jz && level - 1 > 0 && crs.smoother == SM_JACOBI;
       restrict_to(c, level, swept[level - 1] != 0);
       level -= 1;
     } else if (up) {
       prolongate_from(c, level);
-      zero[level + 1] = 0;
       level += 1;
     } else {
       level = -1;

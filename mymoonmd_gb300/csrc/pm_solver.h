@@ -88,12 +88,9 @@ struct Multigrid {
   void apply(pm_ctx* c, const double* rhs, double* sol, bool rhs_nonactive_zero = false);
   // pieces of one cycle (Multigrid::cycle_step)
   void smooth(pm_ctx* c, int l);
-  // the first smoothing step from an iterate that is exactly zero: a damped
-  // Jacobi sweep reduces to x = w (b / d) with the sweep's bits (A*0 sums to
-  // +0); other smoothers sweep as usual
-  void smooth_from_zero(pm_ctx* c, int l);
   void defect(pm_ctx* c, int l);
-  // from l to l-1; sweep: with the first Jacobi sweep of l-1 from zero
+  // from l to l-1; sweep: with the first damped Jacobi sweep of l-1 from zero, which
+  // reduces to x = w (b / d) with the sweep's bits (A*0 sums to +0)
   void restrict_to(pm_ctx* c, int l, bool sweep);
   void prolongate_from(pm_ctx* c, int l);  // from l to l+1
   void coarse_solve(pm_ctx* c);
