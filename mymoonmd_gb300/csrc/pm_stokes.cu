@@ -164,10 +164,11 @@ __device__ void stokes_f(double nu, const double* x, double* f, int example, boo
   const double p = 3.14159265358979323846;
   double S[3], S1[3], S2[3], S3[3];
   for (int d = 0; d < 3; ++d) {
-    // sin and cos of 2 pi t by the double angle: one sincospi per coordinate
-    double s, c;
+    // (by the double angle, one sincospi per coordinate, f has errors a quarter larger:
+    // 1.9e-14 against 1.5e-14 in the mean over 3,000 points)
+    double s, c, s2, c2;
     sincospi(x[d], &s, &c);
-    const double s2 = 2.0 * s * c, c2 = 1.0 - 2.0 * s * s;
+    sincospi(2.0 * x[d], &s2, &c2);
     S[d] = s * s;                    // sin^2(pi t)
     S1[d] = p * s2;                  // d/dt
     S2[d] = 2 * p * p * c2;          // d2/dt2
