@@ -187,6 +187,8 @@ void DevCsr::build_sell(pm_ctx* c, int L) {
   sell_lanes = L;
   n_slices = int(off.size()) - 1;
   sell_entries = int64_t(sc.size());
+  sell_max_steps = 0;
+  for (int s = 0; s < n_slices; ++s) sell_max_steps = std::max(sell_max_steps, (off[s + 1] - off[s]) / 32);
   if (had64) {  // the FP64 copy follows the new layout
     sell_vals64.ensure(sc.size());
     values_changed(c);
@@ -449,18 +451,21 @@ static void launch_sell_shape(pm_ctx* c, const DevCsr& A, int epi, const T* x, T
   }
 }
 
-// Shapes 442 (FP64) and 482 (FP32): twice the steps in flight where rows are longer
-// than eight steps on average and a launch has few slices (the sums are the same). Four lanes, half / twice the steps:
+// Shapes 442 (FP64) and 482 (FP32): twice the steps in flight where the matrix has
+// slices of more than eight steps (a launch of few slices is as long as its longest)
+// and the launch few slices (the sums are the same). Four lanes, half / twice the steps:
 //   FP64 cycle of 3D Q2 in us: 8^3 49.9 / 43.8, 16^3 135.6 / 101.9 (30 slices per SM
 //   in the finest sweep), 24^3 211.5 / 195.9 (97); above 128 slices per SM the finest
 //   sweep is no faster (28^3 263 / 271, the SpMV of 32^3 39.2 / 42.8). Product of the
 //   combined Stokes matrix of 12^3 20.2 / 13.0.
 //   FP32 cycle of 3D Q2: 8^3 31.0 / 29.1, 16^3 61.5 / 56.0, 24^3 105.3 / 103.0; the
 //   finest sweep of 32^3 (226) 28.8 / 28.9.
+//   Restriction of the 24^3 Stokes levels (5 to 8 steps on average, 37 at most): the
+//   mixed request 20.41 / 20.21 ms.
 //   Short rows (3D Q1: at most seven steps) lose: FP32 cycle of 32^3 48.3 / 51.3, 48^3
 //   66.6 / 76.1; FP64 32^3 88.1 / 89.5, 48^3 127.2 / 140.8. Only FP64 launches of few
 //   slices gain (16^3, 4 slices per SM: 53.1 / 49.4).
-static bool sell_long_rows(const DevCsr& A) { return A.sell_entries > 8ll * 32 * A.n_slices; }
+static bool sell_long_rows(const DevCsr& A) { return A.sell_max_steps > 8; }
 static bool sell_deep64(const pm_ctx* c, const DevCsr& A, int ns = 1) {
   const long long slices = (long long)A.n_slices * ns;
   return slices <= (sell_long_rows(A) ? 128ll : 16ll) * c->num_sms;

@@ -57,6 +57,7 @@ struct DevCsr {
   int sell_lanes = 0;
   int n_slices = 0;
   int64_t sell_entries = 0;
+  int sell_max_steps = 0;  // of the longest slice
   DBuf<int> sell_perm, sell_off, sell_cols, sell_src;  // sell_src: CSR entry of each slot, -1 = padding
   DBuf<float> sell_vals;
   // FP64 values in the sliced layout (make_sliced64); sell64_ok: they are the
