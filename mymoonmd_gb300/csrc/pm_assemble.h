@@ -30,7 +30,6 @@ __device__ __forceinline__ double gather_entry(const int* __restrict__ idx, cons
   return s;
 }
 
-// reference-element tables of a Qk element on a tensor Gauss rule
 // 1D tables of a tensor-product element (Q1, Q2) on its Gauss rule, K1 = k + 1
 // basis functions: M_ij = sum_q w phi_i phi_j, S_ij = sum_q w phi_i' phi_j',
 // C_ij = sum_q w phi_i phi_j' (row-major K1 x K1), phiw[q K1 + i] = w_q phi_i(q)
@@ -38,6 +37,7 @@ __device__ __forceinline__ double gather_entry(const int* __restrict__ idx, cons
 struct Tables1d {
   double M[9], S[9], C[9], phiw[12], xi[4];
 };
+// reference-element tables (Qk on a tensor Gauss rule, Pk on a tetrahedral one)
 struct RefTables {
   int dim = 0, nb = 0, nq = 0;
   std::vector<double> w, xi, phi, dphi;

@@ -1092,6 +1092,16 @@ static void allow_nodal_patch_smem();
 bool DevNodalVanka::build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vector<int>& vp,
                                const std::vector<int>& vi, const std::vector<int>& color, int n_colors) {
   if (n_colors > 32 || max_nodes > kNodalMaxNodes) return false;
+  // the other components' rows: the first one's columns, moved to their own component
+  for (int k = 1; k < 3; ++k)
+    for (int i = 0; i < nu; ++i) {
+      const int r0 = S.row_ptr[i], len = S.row_ptr[i + 1] - r0, q0 = S.row_ptr[k * nu + i];
+      if (S.row_ptr[k * nu + i + 1] - q0 != len) return false;
+      for (int e = 0; e < len; ++e) {
+        const int col = S.cols[r0 + e];
+        if (S.cols[q0 + e] != (col < nu ? col + k * nu : col)) return false;
+      }
+    }
   constexpr int C = 8, Lanes = 4;
   std::vector<int> voff(size_t(np) + 1, 0), ioff(size_t(np) + 1, 0), ch0(size_t(np) + 1, 0), hptr(size_t(np) + 1, 0),
       hnv(np), self(np), halo, src;
@@ -1123,15 +1133,6 @@ bool DevNodalVanka::build_pack(pm_ctx* c, const pmsetup::Csr& S, const std::vect
     lenp.assign(m, 0);
     for (int a = 0; a < m; ++a) {
       const int r0 = S.row_ptr[nd[a]], r1 = S.row_ptr[nd[a] + 1];
-      // the other components' rows: the same columns, moved to their own component
-      for (int k = 1; k < 3; ++k) {
-        const int q0 = S.row_ptr[k * nu + nd[a]];
-        if (S.row_ptr[k * nu + nd[a] + 1] - q0 != r1 - r0) return false;
-        for (int e = 0; e < r1 - r0; ++e) {
-          const int col = S.cols[r0 + e];
-          if (S.cols[q0 + e] != (col < nu ? col + k * nu : col)) return false;
-        }
-      }
       for (int k = r0; k < r1; ++k) {
         const int col = S.cols[k];
         if (col < nu) {
