@@ -416,7 +416,7 @@ def run_ours(args, w, rank, world, local, pg):
                                 "colour's patches from their packed rows, their Schur-complement local solves "
                                 "and the update; all colours of both fine levels)"
                                 if stokes else
-                                "sell_kernel<4,16,PIPE,EPI_JACOBI>: finest-level damped Jacobi sweep in FP32 "
+                                "sell_kernel<4,8,PIPE,EPI_JACOBI>: finest-level damped Jacobi sweep in FP32 "
                                 "on the sliced-ELL copy (the largest share of a mixed request's GPU time)"),
                      "achieved": round(achieved, 1) if achieved else None, "peak": hbm_peak,
                      "unit": "GB/s", "frac": round(achieved / hbm_peak, 3) if achieved else None,
